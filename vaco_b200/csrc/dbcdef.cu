@@ -539,6 +539,10 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         __syncthreads();
         deblock_filter<0, NT>(a, ssx, ssy, smem, s_list, s_count, s_str);
         deblock_filter<1, NT>(a, ssx, ssy, smem, s_list + kListTotal, s_count + 4, s_str);
+    } else {
+        // the sample check above reads every staged sample, the sentinel
+        // phase below overwrites some
+        __syncthreads();
     }
 
     // ---- stripe-boundary rows of the deblocked picture for restoration:
