@@ -189,17 +189,9 @@ namespace cdefk {
 // ---------------------------------------------------------------- two pixels per register
 //
 // filter_px() for a horizontal pair of pixels held as two 16-bit lanes of one
-// 32-bit word (low lane = left pixel), using the sm_90+ packed min/max.  Every
-// per-lane quantity below stays in [0, 65535], so plain 32-bit adds and
-// subtracts never carry or borrow across lanes:
-//   hi = max(v, cur), lo = min(v, cur), |d| = hi - lo, d+ = hi - cur
-//   m  = t - min(|d| >> s, t)               (= max(0, t - (|d| >> s)))
-//   c  = min(|d|, m), c+ = min(c, d+)       (c+: constrain's positive part)
-//   acc+ += tap * c+, acc += tap * c        (each <= 24 * 240 = 5760), and
-//   at the end acc- = acc - acc+ (the negative parts' sum)
-// Output: with pos/neg the non-negative parts of acc+ - acc-,
-//   r+ = (pos + 8) >> 4, r- = (neg + 8) >> 4  (vaco's signed rounding)
-//   out = min(max(cur + r+, mn + r-) - r-, mx) = clamp(cur + r+ - r-, mn, mx).
+// 32-bit word (low lane = left pixel).  Two forms with equal results: one in
+// 16-bit integers (any bit depth) and one in half-precision arithmetic that
+// is exact for samples of up to 10 bits (see HalfBlock).
 __device__ __forceinline__ uint32_t vmin2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -210,73 +202,24 @@ __device__ __forceinline__ uint32_t vmax2(uint32_t a, uint32_t b) {
     asm("max.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-
-// Per-block tap description for the pair filter.
-struct PairBlock {
-    int16_t off[6];       // tap offsets (samples): primary d0,d1; dir+2 d0,d1; dir+6 d0,d1
-    uint16_t pri, sec;
-    uint8_t pri_shift, sec_shift, pt0, pt1;
-};
-
-__device__ __forceinline__ PairBlock make_pair_block(int dir, int pri, int sec, int damping, int shift, int pitch) {
-    PairBlock f;
-    f.off[0] = (int16_t)dir_offset<0>(dir, pitch);
-    f.off[1] = (int16_t)dir_offset<1>(dir, pitch);
-    f.off[2] = (int16_t)dir_offset<0>((dir + 2) & 7, pitch);
-    f.off[3] = (int16_t)dir_offset<1>((dir + 2) & 7, pitch);
-    f.off[4] = (int16_t)dir_offset<0>((dir + 6) & 7, pitch);
-    f.off[5] = (int16_t)dir_offset<1>((dir + 6) & 7, pitch);
-    f.pri = (uint16_t)pri;
-    f.sec = (uint16_t)sec;
-    f.pri_shift = (uint8_t)(pri ? max(0, damping - ilog2u(pri)) : 0);
-    f.sec_shift = (uint8_t)(sec ? max(0, damping - ilog2u(sec)) : 0);
-    const bool odd = ((pri >> shift) & 1) != 0;
-    f.pt0 = odd ? 3 : 4;
-    f.pt1 = odd ? 3 : 2;
-    return f;
+__device__ __forceinline__ uint32_t vmins2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("min.s16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
 }
-
-// The pair of samples starting at sample index `i` (any parity) of a plane
-// staged at 4-byte alignment: two aligned word loads and a byte permute.
-struct PairTap {
-    const uint32_t* w;  // aligned word holding sample i & ~1
-    uint32_t sel;       // byte selector: 0x3210 (i even) or 0x5432 (i odd)
-};
-
-__device__ __forceinline__ PairTap pair_tap(const uint16_t* base, int i) {
-    PairTap t;
-    t.w = reinterpret_cast<const uint32_t*>(base + (i & ~1));
-    t.sel = (i & 1) ? 0x5432u : 0x3210u;
-    return t;
+__device__ __forceinline__ uint32_t vmaxs2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.s16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
 }
-
-__device__ __forceinline__ uint32_t load_pair(const PairTap& t, int word_off) {
-    return __byte_perm(t.w[word_off], t.w[word_off + 1], t.sel);
-}
-
-// A tap whose pair is one aligned word: of the plane itself when the pair
-// starts on an even sample, of a copy shifted by one sample when it starts
-// on an odd one.
-struct WordTap {
-    const uint32_t* w;
-};
-
-__device__ __forceinline__ uint32_t load_pair(const WordTap& t, int word_off) { return t.w[word_off]; }
-
-template <bool MASK_MAX>
-__device__ __forceinline__ void pair_tap_step(uint32_t v, uint32_t cur, uint32_t t2, int s, uint32_t smask, uint32_t w,
-                                              uint32_t& accp, uint32_t& acct, uint32_t& mn, uint32_t& mx) {
-    const uint32_t hi = vmax2(v, cur), lo = vmin2(v, cur);
-    const uint32_t ad = hi - lo;
-    const uint32_t sh = (ad >> s) & smask;
-    const uint32_t m = t2 - vmin2(sh, t2);
-    const uint32_t c = vmin2(ad, m);
-    const uint32_t cp = vmin2(c, hi - cur);
-    accp += w * cp;
-    acct += w * c;
+// Minimum and maximum over the available taps: the sentinel is the largest
+// value to an unsigned minimum and negative to a signed maximum, so neither
+// ever picks it (samples are below 2^12).
+__device__ __forceinline__ void tap_range(uint32_t v, uint32_t& mn, uint32_t& mx) {
     mn = vmin2(mn, v);
-    mx = vmax2(mx, MASK_MAX ? (v & 0x3FFF3FFFu) : v);
+    mx = vmaxs2(mx, v);
 }
+static_assert(kSent > 0x0FFF && (kSent & 0x8000), "tap_range relies on it");
 
 // Which tap sets a tile's blocks use.  vaco's filter_block clamps the result
 // to the min/max of every available tap, but when only one tap set has a
@@ -287,31 +230,90 @@ __device__ __forceinline__ void pair_tap_step(uint32_t v, uint32_t cur, uint32_t
 // makes every constrain() of its set 0.  So the taps of a set whose preset
 // strength is zero are skipped altogether (pri_on / sec_on, uniform over a
 // tile), bit-exactly: the clamp over the remaining set is a no-op.
+//
+// The taps of filter_pair() are 12 functions of the row's word offset, in the
+// order +off[0], -off[0], +off[1], ...: primary d0, d1, then dir+2 d0, d1,
+// then dir+6 d0, d1.
 
-// Filter the pixel pair whose left sample is at `s` (4-byte aligned).  `taps`
-// are the 12 tap positions of the block for this lane, `row` the word offset
-// of the current row relative to the block's first row.  MASK_MAX: the tile
-// touches a plane edge, so sentinel samples must not raise the maximum.
-template <bool MASK_MAX, class Tap>
-__device__ __forceinline__ uint32_t filter_pair(uint32_t cur, const Tap* taps, int row, const PairBlock& f,
+// ---- integer form
+//
+// Every per-lane quantity stays in [0, 65535], so plain 32-bit adds and
+// subtracts never carry or borrow across lanes:
+//   hi = max(v, cur), |d| = hi - min(v, cur), d+ = hi - cur
+//   c  = max(min(|d|, t - (|d| >> s)), 0), c+ = min(c, d+)  (constrain and its
+//        positive part; t - x is formed as (t + 1) + ~x, one fused
+//        add-min-clamp on signed lanes.  A sentinel's |d| is above 2^15, i.e.
+//        negative there, which clamps to the 0 it has to give)
+//   acc+ += tap * c+, acc += tap * c        (each <= 24 * 240 = 5760), and
+//   at the end acc- = acc - acc+ (the negative parts' sum)
+// Output: with pos/neg the non-negative parts of acc+ - acc-,
+//   r+ = (pos + 8) >> 4, r- = (neg + 8) >> 4  (vaco's signed rounding)
+//   out = min(max(cur + r+, mn + r-) - r-, mx) = clamp(cur + r+ - r-, mn, mx).
+struct PairBlock {
+    int16_t off[6];       // tap offsets (samples): primary d0,d1; dir+2 d0,d1; dir+6 d0,d1
+    uint16_t pri, sec;
+    uint8_t pri_shift, sec_shift, pt0, pt1;
+};
+
+template <class Block>
+__device__ __forceinline__ void set_offsets(Block& f, int dir, int pitch) {
+    f.off[0] = (int16_t)dir_offset<0>(dir, pitch);
+    f.off[1] = (int16_t)dir_offset<1>(dir, pitch);
+    f.off[2] = (int16_t)dir_offset<0>((dir + 2) & 7, pitch);
+    f.off[3] = (int16_t)dir_offset<1>((dir + 2) & 7, pitch);
+    f.off[4] = (int16_t)dir_offset<0>((dir + 6) & 7, pitch);
+    f.off[5] = (int16_t)dir_offset<1>((dir + 6) & 7, pitch);
+}
+
+__device__ __forceinline__ void make_block(PairBlock& f, int dir, int pri, int sec, int damping, int shift,
+                                           int pitch) {
+    set_offsets(f, dir, pitch);
+    f.pri = (uint16_t)pri;
+    f.sec = (uint16_t)sec;
+    f.pri_shift = (uint8_t)(pri ? max(0, damping - ilog2u(pri)) : 0);
+    f.sec_shift = (uint8_t)(sec ? max(0, damping - ilog2u(sec)) : 0);
+    const bool odd = ((pri >> shift) & 1) != 0;
+    f.pt0 = odd ? 3 : 4;
+    f.pt1 = odd ? 3 : 2;
+}
+
+struct PairSet {  // one tap set's strength and shift
+    uint32_t t1, mask;
+    int s;
+    __device__ __forceinline__ PairSet(uint32_t t, int shift)
+        : t1((t + 1) * 0x10001u), mask((0xFFFFu >> shift) * 0x10001u), s(shift) {}
+};
+
+__device__ __forceinline__ void tap_step(uint32_t v, uint32_t cur, uint32_t ncur, const PairSet& k, uint32_t w,
+                                         uint32_t& accp, uint32_t& acct, uint32_t& mn, uint32_t& mx) {
+    const uint32_t hi = vmax2(v, cur);
+    const uint32_t ad = hi - vmin2(v, cur);
+    const uint32_t c = __viaddmin_s16x2_relu(k.t1, ~((ad >> k.s) & k.mask), ad);
+    accp += w * __viaddmin_u16x2(hi, ncur, c);
+    acct += w * c;
+    tap_range(v, mn, mx);
+}
+
+// Filters the pair `cur`; tap(k, row) is the pair at tap k, `row` the word
+// offset of the current row from the taps' first row.
+template <class Taps>
+__device__ __forceinline__ uint32_t filter_pair(uint32_t cur, const Taps& tap, int row, const PairBlock& f,
                                                 bool pri_on, bool sec_on) {
-    const uint32_t tp = f.pri | ((uint32_t)f.pri << 16), ts = f.sec | ((uint32_t)f.sec << 16);
-    const uint32_t pm = (0xFFFFu >> f.pri_shift) * 0x10001u, sm = (0xFFFFu >> f.sec_shift) * 0x10001u;
+    const PairSet kp(f.pri, f.pri_shift), ks(f.sec, f.sec_shift);
+    const uint32_t ncur = ~cur + 0x00010001u - (((cur & 0xFFFFu) == 0) ? 0x00010000u : 0u);  // -cur per lane
     uint32_t accp = 0, acct = 0, mn = cur, mx = cur;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const uint32_t wp = k ? f.pt1 : f.pt0, ws = 2 - k;
         if (pri_on) {
-            pair_tap_step<MASK_MAX>(load_pair(taps[2 * k], row), cur, tp, f.pri_shift, pm, wp, accp, acct, mn, mx);
-            pair_tap_step<MASK_MAX>(load_pair(taps[2 * k + 1], row), cur, tp, f.pri_shift, pm, wp, accp, acct, mn, mx);
+            tap_step(tap(2 * k, row), cur, ncur, kp, wp, accp, acct, mn, mx);
+            tap_step(tap(2 * k + 1, row), cur, ncur, kp, wp, accp, acct, mn, mx);
         }
         if (sec_on) {
-            pair_tap_step<MASK_MAX>(load_pair(taps[4 + 2 * k], row), cur, ts, f.sec_shift, sm, ws, accp, acct, mn, mx);
-            pair_tap_step<MASK_MAX>(load_pair(taps[4 + 2 * k + 1], row), cur, ts, f.sec_shift, sm, ws, accp, acct, mn,
-                                    mx);
-            pair_tap_step<MASK_MAX>(load_pair(taps[8 + 2 * k], row), cur, ts, f.sec_shift, sm, ws, accp, acct, mn, mx);
-            pair_tap_step<MASK_MAX>(load_pair(taps[8 + 2 * k + 1], row), cur, ts, f.sec_shift, sm, ws, accp, acct, mn,
-                                    mx);
+            tap_step(tap(4 + 2 * k, row), cur, ncur, ks, ws, accp, acct, mn, mx);
+            tap_step(tap(4 + 2 * k + 1, row), cur, ncur, ks, ws, accp, acct, mn, mx);
+            tap_step(tap(8 + 2 * k, row), cur, ncur, ks, ws, accp, acct, mn, mx);
+            tap_step(tap(8 + 2 * k + 1, row), cur, ncur, ks, ws, accp, acct, mn, mx);
         }
     }
     const uint32_t accn = acct - accp;
@@ -319,6 +321,119 @@ __device__ __forceinline__ uint32_t filter_pair(uint32_t cur, const Tap* taps, i
     const uint32_t rp = ((accp - both + 0x00080008u) >> 4) & 0x0FFF0FFFu;
     const uint32_t rn = ((accn - both + 0x00080008u) >> 4) & 0x0FFF0FFFu;
     return vmin2(vmax2(cur + rp, mn + rn) - rn, mx);
+}
+
+// ---- half-precision form, samples of up to 10 bits
+//
+// The bits of a 16-bit integer n <= 2048 are those of the half-precision
+// number n 2^-24: up to 1023 as a subnormal, then as the first normal numbers,
+// which have the same spacing.  So a word of two samples is a pair of halves
+// as it is, in units of 2^-24, and sums and differences are exact while they
+// stay within 2048 units.  Per tap, with s the set's shift and t its strength:
+//   d  = v - cur                       exact
+//   e  = 2 |d| + (1 - 2^s)             exact (at most 2047)
+//   m  = max(t - e / 2^(s+1), 0)       one fused multiply-add, which rounds to
+//        whole units: with |d| = q 2^s + r, e / 2^(s+1) = q + (2r + 1 - 2^s) /
+//        2^(s+1), whose fraction lies strictly inside (-1/2, 1/2), so m is
+//        max(t - (|d| >> s), 0) for every |d|
+//   c  = min(|d|, m) with d's sign     constrain(d)
+//   acc += tap * c                     exact (at most 12 * 60 + 12 * 16 = 912)
+// Four of these run on the FMA pipe and, with the min and max of the taps,
+// three on the ALU pipe (the absolute values are operand modifiers), against
+// about eleven mostly on the ALU pipe in integers.  A shift of 10 or more
+// makes |d| >> s zero for every |d| < 1024, as a shift of 10 does.  The
+// sentinel reads as -2.0, far above 2^11 units: m is 0 for every s <= 10.
+// The fused kernel took 145 us and 100.7 M warp instructions per 4K 10-bit
+// frame with integer taps, 115 us and 78.4 M with these.
+struct __align__(16) HalfBlock {
+    uint32_t pt, pk1, pk2;  // primary set: t, 1 - 2^s, -2^-(s+1), both lanes
+    uint32_t st, sk1, sk2;  // secondary set
+    uint32_t w0, w1;        // primary tap weights at distances 1 and 2
+    int16_t off[6];
+};
+
+__device__ __forceinline__ uint32_t h2(uint32_t bits) { return bits * 0x10001u; }
+
+__device__ __forceinline__ void half_set(int t, int s, uint32_t& ht, uint32_t& k1, uint32_t& k2) {
+    s = min(s, 10);
+    ht = h2((uint32_t)t);
+    k1 = s ? h2(0x8000u | ((1u << s) - 1)) : 0u;   // -(2^s - 1) units
+    k2 = h2(0x8000u | (uint32_t)(14 - s) << 10);   // -2^-(s+1): exponent 15 - (s + 1)
+}
+
+__device__ __forceinline__ void make_block(HalfBlock& f, int dir, int pri, int sec, int damping, int shift,
+                                           int pitch) {
+    set_offsets(f, dir, pitch);
+    half_set(pri, pri ? max(0, damping - ilog2u(pri)) : 0, f.pt, f.pk1, f.pk2);
+    half_set(sec, sec ? max(0, damping - ilog2u(sec)) : 0, f.st, f.sk1, f.sk2);
+    const bool odd = ((pri >> shift) & 1) != 0;
+    f.w0 = odd ? 0x42004200u : 0x44004400u;  // 3.0 : 4.0
+    f.w1 = odd ? 0x42004200u : 0x40004000u;  // 3.0 : 2.0
+}
+
+__device__ __forceinline__ uint32_t hadd2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t hsub2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t hfma2_relu(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t habs2(uint32_t a) {
+    uint32_t d;
+    asm("abs.f16x2 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+__device__ __forceinline__ uint32_t hmin2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("min.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+__device__ __forceinline__ void tap_step_h(uint32_t v, uint32_t cur, uint32_t t, uint32_t k1, uint32_t k2, uint32_t w,
+                                           uint32_t& acc, uint32_t& mn, uint32_t& mx) {
+    const uint32_t d = hsub2(v, cur);
+    const uint32_t e = hfma2(habs2(d), 0x40004000u, k1);
+    const uint32_t c = hmin2(habs2(d), hfma2_relu(e, k2, t));
+    acc = hfma2(c | (d & 0x80008000u), w, acc);
+    tap_range(v, mn, mx);
+}
+
+template <class Taps>
+__device__ __forceinline__ uint32_t filter_pair(uint32_t cur, const Taps& tap, int row, const HalfBlock& f,
+                                                bool pri_on, bool sec_on) {
+    uint32_t acc = 0, mn = cur, mx = cur;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const uint32_t wp = k ? f.w1 : f.w0, ws = k ? 0x3C003C00u : 0x40004000u;  // 1.0 : 2.0
+        if (pri_on) {
+            tap_step_h(tap(2 * k, row), cur, f.pt, f.pk1, f.pk2, wp, acc, mn, mx);
+            tap_step_h(tap(2 * k + 1, row), cur, f.pt, f.pk1, f.pk2, wp, acc, mn, mx);
+        }
+        if (sec_on) {
+            tap_step_h(tap(4 + 2 * k, row), cur, f.st, f.sk1, f.sk2, ws, acc, mn, mx);
+            tap_step_h(tap(4 + 2 * k + 1, row), cur, f.st, f.sk1, f.sk2, ws, acc, mn, mx);
+            tap_step_h(tap(8 + 2 * k, row), cur, f.st, f.sk1, f.sk2, ws, acc, mn, mx);
+            tap_step_h(tap(8 + 2 * k + 1, row), cur, f.st, f.sk1, f.sk2, ws, acc, mn, mx);
+        }
+    }
+    // (8 + sum - (sum < 0)) >> 4 is (|sum| + 8) >> 4 with the sum's sign.  A
+    // result below zero is negative as a signed lane too, so the signed max
+    // with mn >= 0 clamps it.
+    const uint32_t r = (((acc & 0x7FFF7FFFu) + 0x00080008u) >> 4) & 0x07FF07FFu;
+    return vmins2(vmaxs2(hadd2(cur, r | (acc & 0x80008000u)), mn), mx);
 }
 
 }  // namespace cdefk

@@ -45,8 +45,11 @@ constexpr int kHalo = 8;
 // 3 x 340), 1 = chroma size 8 (2 x 340), 2 = luma size 8, 3 = luma size 16.
 __constant__ int c_list_off[4] = {0, 1020, 1700, 2040};
 constexpr int kListTotal = 2380;
-// Rows of the luma CDEF window (th + 4) kept as odd-aligned pairs.
+// Rows of the luma CDEF window (th + 4) kept as odd-aligned pairs, and the
+// words of luma's and both 4:2:0 chroma planes' (see shift_copy()).
 constexpr int kShiftRows = 64 + 4;
+constexpr bool kShiftChroma = true;
+constexpr int kShiftWords = kShiftRows * (64 + 2 * kHalo) / 2 + 2 * (32 + 2 * kHalo) * (32 + 2 * kHalo) / 2;
 
 // Side-information window of a tile: cells [mi_r0 - kWinTop, +kWinRows) x
 // [mi_c0 - kWinLeft, +kWinCols) of the luma maps, and the same shape around
@@ -112,108 +115,120 @@ struct DbCdefArgs {
     size_t plane_off[3];        // shared-memory offset (samples) of each staged plane
 };
 
-// CDEF output of one plane tile from the staged (deblocked) samples: one warp
-// filters block row br; lane l owns pixel pairs at tile column 2*(l % ppr),
-// rows l / ppr + RPI*j.  PITCH is the staged pitch, BH the block height.
+// The taps of one lane as words of the staged plane: a pair that starts on an
+// even sample is one aligned word of the plane, one that starts on an odd
+// sample one word of a copy shifted by one sample.
+struct WordTaps {
+    const uint32_t* w[12];
+    __device__ __forceinline__ uint32_t operator()(int k, int row) const { return w[k][row]; }
+};
+// The same without a shifted copy: two aligned words and a byte permute.
+struct PairTaps {
+    const uint32_t* w[12];  // aligned word holding sample i & ~1
+    uint32_t sel[12];       // 0x3210 (i even) or 0x5432 (i odd)
+    __device__ __forceinline__ uint32_t operator()(int k, int row) const {
+        return __byte_perm(w[k][row], w[k][row + 1], sel[k]);
+    }
+};
+
+// CDEF output of block row br of planes p0 .. p0 + NPL - 1 (both chroma planes
+// share their blocks' parameters) from the staged (deblocked) samples `t` of
+// plane p0; the next plane's are `plane_words` words on.  One warp; lane l
+// owns pixel pairs at tile column 2*(l % ppr), rows l / ppr + RPI*j.  PITCH is
+// the staged pitch, BH the block height.
 // pri_on / sec_on: the tile preset's primary / secondary strength is
 // non-zero; with neither, every sample stays as it is.
-// SHIFT (luma): s1 holds the tile's luma pairs that start on odd samples,
-// kShiftRows rows from row kHalo - 2 on the staged pitch, so every tap is a
-// single aligned word.
-template <int PITCH, int BH, int RPI, bool EDGE, bool SHIFT>
-__device__ __forceinline__ void filter_pairs(const uint16_t* t, const uint32_t* s1, const DevPlane& d,
-                                             const DirectPlane* D, int px0, int py0, int tw, const uint8_t* active,
-                                             const PairBlock* blocks, bool pri_on, bool sec_on, int br, int lane,
-                                             int sx) {
-    const int ppr = 32 / RPI;              // pairs per row
-    const int lp = lane % ppr, lr = lane / ppr;
-    const int x = 2 * lp;
-    if (x >= tw) return;
-    const int bx = x >> (3 - sx);
-    const int gx = px0 + x;
-    const bool col_in = gx < d.width;
+// SHIFT: the pairs that start on odd samples are at s1, rows from row kHalo-2
+// on the staged pitch, planes at the same distance.
+template <int PITCH, int BH, int RPI, int NPL, bool SHIFT, bool DIRECT, class Block>
+__device__ __forceinline__ void filter_block_row(const DbCdefArgs& a, int p0, const uint16_t* t, const uint32_t* s1,
+                                                 int plane_words, int px0, int py0, const uint8_t* active,
+                                                 const Block* blocks, bool pri_on, bool sec_on, int br, int lane,
+                                                 int sx) {
+    constexpr int ppr = 32 / RPI;          // pairs per row: the tile is 2 ppr samples wide
+    const int x = 2 * (lane % ppr), lr = lane / ppr;
     const int r0 = br * BH;
-    if (py0 + r0 >= d.height) return;
-    const int rows_here = min(BH, d.height - (py0 + r0));
-    const int b = br * 8 + bx;
+    const int gx = px0 + x;
+    const int width = a.dst[p0].width, height = a.dst[p0].height;
+    if (py0 + r0 >= height) return;
+    const bool col_in = gx < width;
+    const int rows_here = min(BH, height - (py0 + r0));
+    const int b = br * 8 + (x >> (3 - sx));
     const int base_i = (kHalo + r0 + lr) * PITCH + kHalo + x;  // left sample, first row of this lane
-    uint32_t* o = reinterpret_cast<uint32_t*>(d.data + (long)(py0 + r0 + lr) * d.stride + gx);
-    const long ostride = (long)d.stride * RPI / 2;  // words per RPI rows
-    const uint32_t* cw = reinterpret_cast<const uint32_t*>(t + base_i);
-    // The final output too, for a plane without restoration (DirectPlane).
-    uint16_t* od = nullptr;
-    int od_rows = 0;
-    bool od_pair = false;
-    if (D && D->out.data && gx < D->out.width) {
-        od = D->out.data + (long)(py0 + r0 + lr) * D->out.stride + gx;
-        od_rows = min(BH, D->out.height - (py0 + r0));
-        od_pair = gx + 1 < D->out.width;
-    }
-    auto put = [&](int j, uint32_t v) {
-        if (od && lr + RPI * j < od_rows) {
-            uint16_t* q = od + (long)j * RPI * D->out.stride;
-            if (od_pair) *reinterpret_cast<uint32_t*>(q) = v;
-            else *q = (uint16_t)v;
+    const uint32_t* t32 = reinterpret_cast<const uint32_t*>(t);
+    const uint32_t* cw = t32 + (base_i >> 1);
+    // Runs out(word offset, value) over the lane's rows of every plane.
+    auto rows = [&](auto&& value) {
+#pragma unroll 1  // smaller code: the fused kernel is sensitive to instruction fetch
+        for (int pl = 0; pl < NPL; ++pl) {
+            const DevPlane& d = a.dst[p0 + pl];
+            uint32_t* o = reinterpret_cast<uint32_t*>(d.data + (long)(py0 + r0 + lr) * d.stride + gx);
+            const long ostride = (long)d.stride * RPI / 2;  // words per RPI rows
+            // The final output too, for a plane without restoration (DirectPlane).
+            uint16_t* od = nullptr;
+            int od_rows = 0;
+            bool od_pair = false;
+            if (DIRECT) {
+                const DevPlane& D = a.direct[p0 + pl].out;
+                if (D.data && gx < D.width) {
+                    od = D.data + (long)(py0 + r0 + lr) * D.stride + gx;
+                    od_rows = min(BH, D.height - (py0 + r0));
+                    od_pair = gx + 1 < D.width;
+                }
+            }
+#pragma unroll 1
+            for (int j = 0; j < BH / RPI; ++j) {
+                const uint32_t v = value(pl * plane_words + j * (RPI * PITCH / 2));
+                if (col_in && lr + RPI * j < rows_here) o[j * ostride] = v;
+                if (DIRECT && od && lr + RPI * j < od_rows) {
+                    uint16_t* q = od + (long)j * RPI * a.direct[p0 + pl].out.stride;
+                    if (od_pair) *reinterpret_cast<uint32_t*>(q) = v;
+                    else *q = (uint16_t)v;
+                }
+            }
         }
     };
     if ((pri_on || sec_on) && active[b]) {
-        const PairBlock f = blocks[b];
+        const Block f = blocks[b];
         if (SHIFT) {
-            const uint32_t* t32 = reinterpret_cast<const uint32_t*>(t);
             auto word_tap = [&](int i) {  // i: staged index of the pair's first sample
-                return WordTap{(i & 1) ? s1 + ((i >> 1) - (kHalo - 2) * (PITCH / 2)) : t32 + (i >> 1)};
+                return (i & 1) ? s1 + ((i >> 1) - (kHalo - 2) * (PITCH / 2)) : t32 + (i >> 1);
             };
-            WordTap taps[12];
+            WordTaps taps;
 #pragma unroll
             for (int k = 0; k < 6; ++k) {
-                taps[2 * k] = word_tap(base_i + f.off[k]);
-                taps[2 * k + 1] = word_tap(base_i - f.off[k]);
+                taps.w[2 * k] = word_tap(base_i + f.off[k]);
+                taps.w[2 * k + 1] = word_tap(base_i - f.off[k]);
             }
-#pragma unroll 1  // smaller code: the fused kernel is sensitive to instruction fetch
-            for (int j = 0; j < BH / RPI; ++j) {
-                const int woff = j * RPI * PITCH / 2;
-                const uint32_t v = filter_pair<EDGE>(cw[woff], taps, woff, f, pri_on, sec_on);
-                if (col_in && lr + RPI * j < rows_here) o[j * ostride] = v;
-                put(j, v);
-            }
+            rows([&](int row) { return filter_pair(cw[row], taps, row, f, pri_on, sec_on); });
         } else {
-            PairTap taps[12];
+            PairTaps taps;
 #pragma unroll
             for (int k = 0; k < 6; ++k) {
-                taps[2 * k] = pair_tap(t, base_i + f.off[k]);
-                taps[2 * k + 1] = pair_tap(t, base_i - f.off[k]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int i = base_i + (h ? -f.off[k] : f.off[k]);
+                    taps.w[2 * k + h] = t32 + (i >> 1);
+                    taps.sel[2 * k + h] = (i & 1) ? 0x5432u : 0x3210u;
+                }
             }
-#pragma unroll 1  // smaller code: the fused kernel is sensitive to instruction fetch
-            for (int j = 0; j < BH / RPI; ++j) {
-                const int woff = j * RPI * PITCH / 2;
-                const uint32_t v = filter_pair<EDGE>(cw[woff], taps, woff, f, pri_on, sec_on);
-                if (col_in && lr + RPI * j < rows_here) o[j * ostride] = v;
-                put(j, v);
-            }
+            rows([&](int row) { return filter_pair(cw[row], taps, row, f, pri_on, sec_on); });
         }
     } else if (col_in) {
-#pragma unroll
-        for (int j = 0; j < BH / RPI; ++j) {
-            const uint32_t v = cw[j * RPI * PITCH / 2];
-            if (lr + RPI * j < rows_here) o[j * ostride] = v;
-            put(j, v);
-        }
+        rows([&](int row) { return cw[row]; });
     }
 }
 
-template <int PITCH, int BH, int RPI, bool SHIFT>
-__device__ __forceinline__ void filter_pairs_edge(bool edge, const uint16_t* t, const uint32_t* s1, const DevPlane& d,
-                                                  const DirectPlane* D,
-                                                  int px0, int py0, int tw, const uint8_t* active,
-                                                  const PairBlock* blocks, bool pri_on, bool sec_on, int warp,
-                                                  int lane, int sx, int nwarps) {
-    for (int br = warp; br < 8; br += nwarps) {  // 8 block rows
-        if (edge)
-            filter_pairs<PITCH, BH, RPI, true, SHIFT>(t, s1, d, D, px0, py0, tw, active, blocks, pri_on, sec_on, br, lane,
-                                                     sx);
-        else
-            filter_pairs<PITCH, BH, RPI, false, SHIFT>(t, s1, d, D, px0, py0, tw, active, blocks, pri_on, sec_on, br,
-                                                      lane, sx);
+// A staged plane's pairs that start on odd samples, ROWS rows from row
+// kHalo - 2: word w of a row holds samples 2w + 1 and 2w + 2.
+template <int PITCH, int ROWS, int NT>
+__device__ __forceinline__ void shift_copy(const uint16_t* t, uint32_t* shifted) {
+    constexpr int WP = PITCH / 2, W0 = (kHalo - 1) / 2, NW = (PITCH - 2 * kHalo) / 2 + 1;
+    const uint32_t* t32 = reinterpret_cast<const uint32_t*>(t);
+    for (int i = threadIdx.x; i < ROWS * NW; i += NT) {
+        const int r = i / NW, w = W0 + (i - r * NW);
+        const int src = (kHalo - 2 + r) * WP + w;
+        shifted[r * WP + w] = __byte_perm(t32[src], t32[src + 1], 0x5432);
     }
 }
 
@@ -394,7 +409,7 @@ __device__ __forceinline__ void deblock_filter(const DbCdefArgs& a, int ssx, int
 // One 64x64 filter block (tile_x, tile_y) of one frame.  Every thread of the
 // CTA calls it; it ends with all threads past their last shared-memory use
 // only after the caller's next __syncthreads().
-template <int NT, int LAYOUT, bool DIRECT = false>
+template <int NT, int LAYOUT, class Block, bool DIRECT = false>
 __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int tile_y) {
     constexpr int kWarpsNT = NT / 32;
     // chroma subsampling: LAYOUT = ssx | ssy << 1 fixes it at compile time
@@ -402,7 +417,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     const int ssx = LAYOUT < 0 ? a.ssx : (LAYOUT & 1), ssy = LAYOUT < 0 ? a.ssy : (LAYOUT >> 1);
     extern __shared__ __align__(16) uint16_t smem[];
     __shared__ int s_cost[64][8];
-    __shared__ PairBlock s_pair[3][64];
+    __shared__ Block s_block[2][64];  // luma, chroma (U and V share strengths and directions)
     __shared__ uint8_t s_active[64];
     __shared__ int s_count[8];  // list lengths per size class, pass 0 then pass 1
     __shared__ PairStrength s_str[64];  // per loop-filter level, for this frame's sharpness and depth
@@ -413,7 +428,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
             uint32_t list[2 * kListTotal];  // per pass and size class, see seg_entry()
             SideWindow side;
         } db;
-        uint32_t shifted[kShiftRows * (64 + 2 * kHalo) / 2];
+        uint32_t shifted[kShiftWords];
     } s_u;
     uint32_t* s_list = s_u.db.list;
     SideWindow& s_side = s_u.db.side;
@@ -613,18 +628,16 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     }
     __syncthreads();
 
-    // The luma CDEF window's pairs that start on odd samples (rows kHalo-2 ..
+    // The CDEF windows' pairs that start on odd samples (rows kHalo-2 ..
     // kHalo+th+1, first samples on columns kHalo-1 .. kHalo+tw-1), as words
-    // on the staged row pitch, so the pair filter reads every luma tap with
-    // one aligned load.
-    {
-        constexpr int WP = (64 + 2 * kHalo) / 2, W0 = (kHalo - 1) / 2, NW = 64 / 2 + 1;
-        const uint32_t* t32 = reinterpret_cast<const uint32_t*>(smem + a.plane_off[0]);
-        for (int i = tid; i < kShiftRows * NW; i += NT) {
-            const int r = i / NW, w = W0 + (i - r * NW);
-            const int src = (kHalo - 2 + r) * WP + w;
-            s_u.shifted[r * WP + w] = __byte_perm(t32[src], t32[src + 1], 0x5432);
-        }
+    // on the staged row pitch, so the pair filter reads every tap with one
+    // aligned load: luma, and 4:2:0 chroma, whose copies lie as far apart as
+    // the staged planes (the other layouts' do not fit beside luma's).
+    shift_copy<64 + 2 * kHalo, kShiftRows, NT>(smem + a.plane_off[0], s_u.shifted);
+    if (kShiftChroma && a.num_planes > 1 && ssx == 1 && ssy == 1) {
+        uint32_t* sc = s_u.shifted + kShiftRows * (64 + 2 * kHalo) / 2;
+        shift_copy<32 + 2 * kHalo, 32 + 4, NT>(smem + a.plane_off[1], sc);
+        shift_copy<32 + 2 * kHalo, 32 + 4, NT>(smem + a.plane_off[2], sc + (32 + 2 * kHalo) * (32 + 2 * kHalo) / 2);
     }
 
     // Direction search: job j (0..7, spread over the warps) handles direction
@@ -641,14 +654,14 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         }
     }
     __syncthreads();
-    // Per block and plane (one thread each): direction, strengths, checks.
-    for (int i = tid; i < 64 * a.num_planes; i += NT) {
+    // Per block, luma and chroma (one thread each): direction, strengths, checks.
+    for (int i = tid; i < (a.num_planes > 1 ? 128 : 64); i += NT) {
         if (!s_active[i & 63]) continue;
-        const int b = i & 63, p = i >> 6;
+        const int b = i & 63;
+        const bool chroma = i >= 64;
         int dir;
         uint32_t var;
         best_direction(s_cost[b], dir, var);
-        const bool chroma = p != 0;
         int sp = 0, ss = 0;
         if (index < 8) {
             sp = chroma ? a.uv_pri[index] : a.y_pri[index];
@@ -659,45 +672,45 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         const int chosen = primary == 0 ? 0 : chroma ? chroma_direction(dir, ssx, ssy) : dir;
         if (!chroma) primary = adjust_strength(primary, var);
         const int damping = (a.damping + a.shift - (chroma ? 1 : 0)) & 0xFF;
-        // Each plane reports its own failure; the status word keeps the
-        // lowest (block, plane) key, i.e. the first plane vaco would reject.
+        // Luma and chroma report their own failures; the status word keeps the
+        // lowest (block, plane) key, i.e. the first plane vaco would reject
+        // (V, whose parameters are U's, never comes first).
         if (index >= 8 || damping > 12 || primary > (15 << a.shift) || secondary > (4 << a.shift)) {
             const int r = mi_r0 + (b >> 3) * 2, c = mi_c0 + (b & 7) * 2;
-            report_error(a.status, STAGE_CDEF, ((unsigned long long)r * a.mi_cols + c) * 4 + 1 + p,
+            report_error(a.status, STAGE_CDEF, ((unsigned long long)r * a.mi_cols + c) * 4 + 1 + (chroma ? 1 : 0),
                          index >= 8 ? VACO_AV1_MSG_CDEF_STRENGTH_INDEX : VACO_AV1_MSG_CDEF_BLOCK_PARAMS);
         }
-        const PlaneGeom g = plane_geom(p, ssx, ssy);
-        s_pair[p][b] = make_pair_block(chosen, primary, secondary, min(damping, 12), a.shift, g.pitch);
+        const int pitch = plane_geom(chroma ? 1 : 0, ssx, ssy).pitch;
+        make_block(s_block[chroma ? 1 : 0][b], chosen, primary, secondary, min(damping, 12), a.shift, pitch);
     }
     __syncthreads();
 
     // Filtering: pixel pairs (two 16-bit lanes per register), one warp per
-    // block row, lanes across the tile width.
-    for (int p = 0; p < a.num_planes; ++p) {
-        const PlaneGeom g = plane_geom(p, ssx, ssy);
-        const DevPlane& d = a.dst[p];
-        const int px0 = x0 >> g.sx, py0 = y0 >> g.sy;
-        const bool edge = px0 < 2 || py0 < 2 || px0 + g.tw + 2 > d.width || py0 + g.th + 2 > d.height;
-        const uint16_t* tp = smem + a.plane_off[p];
-        // the tile's tap sets, from its preset (uniform over the tile)
-        bool pri_on = true, sec_on = true;
-        if (index < 8) {
-            pri_on = (p ? a.uv_pri[index] : a.y_pri[index]) != 0;
-            sec_on = (p ? a.uv_sec[index] : a.y_sec[index]) != 0;
-        }
-        // tile layouts: 64x64 (luma, 4:4:4 chroma), 32x32 (4:2:0), 32x64 (4:2:2)
-        if (p == 0) {
-            filter_pairs_edge<64 + 2 * kHalo, 8, 1, true>(edge, tp, s_u.shifted, d, DIRECT ? &a.direct[p] : nullptr, px0, py0, g.tw, s_active,
-                                                          s_pair[p], pri_on, sec_on, warp, lane, g.sx, kWarpsNT);
-        } else if (g.tw == 64) {
-            filter_pairs_edge<64 + 2 * kHalo, 8, 1, false>(edge, tp, nullptr, d, DIRECT ? &a.direct[p] : nullptr, px0, py0, g.tw, s_active, s_pair[p],
-                                                           pri_on, sec_on, warp, lane, g.sx, kWarpsNT);
-        } else if (g.th == 32) {
-            filter_pairs_edge<32 + 2 * kHalo, 4, 2, false>(edge, tp, nullptr, d, DIRECT ? &a.direct[p] : nullptr, px0, py0, g.tw, s_active, s_pair[p],
-                                                           pri_on, sec_on, warp, lane, g.sx, kWarpsNT);
-        } else {
-            filter_pairs_edge<32 + 2 * kHalo, 8, 2, false>(edge, tp, nullptr, d, DIRECT ? &a.direct[p] : nullptr, px0, py0, g.tw, s_active, s_pair[p],
-                                                           pri_on, sec_on, warp, lane, g.sx, kWarpsNT);
+    // block row, lanes across the tile width; luma, then both chroma planes.
+    // Tap sets of the tile's preset (uniform over the tile).
+    const bool y_pri_on = index >= 8 || a.y_pri[index] != 0, y_sec_on = index >= 8 || a.y_sec[index] != 0;
+    for (int br = warp; br < 8; br += kWarpsNT)
+        filter_block_row<64 + 2 * kHalo, 8, 1, 1, true, DIRECT>(a, 0, smem + a.plane_off[0], s_u.shifted, 0, x0, y0,
+                                                                s_active, s_block[0], y_pri_on, y_sec_on, br, lane, 0);
+    if (a.num_planes > 1) {
+        const bool c_pri_on = index >= 8 || a.uv_pri[index] != 0, c_sec_on = index >= 8 || a.uv_sec[index] != 0;
+        const uint16_t* tc = smem + a.plane_off[1];
+        const int plane_words = (int)(a.plane_off[2] - a.plane_off[1]) / 2;
+        const int px0 = x0 >> ssx, py0 = y0 >> ssy;
+        // tile layouts: 64x64 (4:4:4), 32x32 (4:2:0), 32x64 (4:2:2)
+        for (int br = warp; br < 8; br += kWarpsNT) {
+            if (ssx == 0)
+                filter_block_row<64 + 2 * kHalo, 8, 1, 2, false, DIRECT>(a, 1, tc, nullptr, plane_words, px0, py0,
+                                                                         s_active, s_block[1], c_pri_on, c_sec_on, br,
+                                                                         lane, ssx);
+            else if (ssy == 1)
+                filter_block_row<32 + 2 * kHalo, 4, 2, 2, kShiftChroma, DIRECT>(
+                    a, 1, tc, s_u.shifted + kShiftRows * (64 + 2 * kHalo) / 2, plane_words, px0, py0, s_active,
+                    s_block[1], c_pri_on, c_sec_on, br, lane, ssx);
+            else
+                filter_block_row<32 + 2 * kHalo, 8, 2, 2, false, DIRECT>(a, 1, tc, nullptr, plane_words, px0, py0,
+                                                                         s_active, s_block[1], c_pri_on, c_sec_on, br,
+                                                                         lane, ssx);
         }
     }
 }
@@ -711,10 +724,10 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
 // DIRECT: a body that also writes the output of planes without restoration
 // (DirectPlane); the code for it measured 3 % slower on frames that have no
 // such plane, so it is a separate body.
-template <int NT, int MIN_CTAS, int LAYOUT, bool DIRECT = false>
+template <int NT, int MIN_CTAS, int LAYOUT, class Block, bool DIRECT = false>
 __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_kernel(DbCdefArgs a) {
     overlap_prologue();
-    dbcdef_tile<NT, LAYOUT, DIRECT>(a, blockIdx.x, blockIdx.y);
+    dbcdef_tile<NT, LAYOUT, Block, DIRECT>(a, blockIdx.x, blockIdx.y);
 }
 
 // Batched form: one CTA per tile of all frames of a batch, frames laid end to
@@ -724,14 +737,14 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_kernel(DbCdefArgs a) {
 // state and the frame record live across the tile and spilled registers: it
 // measured 4 % slower on 4K frames.)  LAYOUT as for dbcdef_tile: a batch
 // whose frames share one chroma layout takes the body compiled for it.
-template <int NT, int MIN_CTAS, int LAYOUT>
+template <int NT, int MIN_CTAS, int LAYOUT, class Block>
 __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_batch_kernel(const DbCdefArgs* __restrict__ frames,
                                                                     const int* __restrict__ tile_prefix, int n) {
     const int f = frame_of_tile(tile_prefix, n, blockIdx.x);
     const DbCdefArgs& a = frames[f];
     const int local = blockIdx.x - tile_prefix[f];
     const int tiles_x = (a.mi_cols + 15) / 16;
-    dbcdef_tile<NT, LAYOUT>(a, local % tiles_x, local / tiles_x);
+    dbcdef_tile<NT, LAYOUT, Block>(a, local % tiles_x, local / tiles_x);
 }
 
 }  // namespace
@@ -806,18 +819,50 @@ cudaError_t dbcdef_kernel_attributes() {
         constexpr int kMaxSmem = 96 * 1024;
         const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
         cudaError_t e = cudaSuccess;
-        for (auto k : {dbcdef_kernel<256, 4, 0>, dbcdef_kernel<256, 4, 1>, dbcdef_kernel<256, 4, 3>,
-                       dbcdef_kernel<256, 4, 0, true>, dbcdef_kernel<256, 4, 1, true>,
-                       dbcdef_kernel<256, 4, 3, true>, dbcdef_kernel<128, 5, 0>, dbcdef_kernel<128, 5, 1>,
-                       dbcdef_kernel<128, 5, 3>})
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, attr, kMaxSmem);
-        for (auto k : {dbcdef_batch_kernel<256, 3, -1>, dbcdef_batch_kernel<256, 3, 0>, dbcdef_batch_kernel<256, 3, 1>,
-                       dbcdef_batch_kernel<256, 3, 3>, dbcdef_batch_kernel<256, 4, -1>, dbcdef_batch_kernel<128, 5, -1>})
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, attr, kMaxSmem);
+        auto optin = [&](auto block) {
+            using B = decltype(block);
+            for (auto k : {dbcdef_kernel<256, 4, 0, B>, dbcdef_kernel<256, 4, 1, B>, dbcdef_kernel<256, 4, 3, B>,
+                           dbcdef_kernel<256, 4, 0, B, true>, dbcdef_kernel<256, 4, 1, B, true>,
+                           dbcdef_kernel<256, 4, 3, B, true>, dbcdef_kernel<128, 5, 0, B>, dbcdef_kernel<128, 5, 1, B>,
+                           dbcdef_kernel<128, 5, 3, B>})
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, attr, kMaxSmem);
+            for (auto k : {dbcdef_batch_kernel<256, 3, -1, B>, dbcdef_batch_kernel<256, 3, 0, B>,
+                           dbcdef_batch_kernel<256, 3, 1, B>, dbcdef_batch_kernel<256, 3, 3, B>,
+                           dbcdef_batch_kernel<256, 4, -1, B>, dbcdef_batch_kernel<128, 5, -1, B>})
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, attr, kMaxSmem);
+        };
+        optin(HalfBlock{});
+        optin(PairBlock{});
         if (e != cudaSuccess) return e;
         g_attr_devices.fetch_or(1ull << dev, std::memory_order_release);
     }
     return cudaSuccess;
+}
+
+// One kernel per chroma layout (4:4:4 and monochrome, 4:2:2, 4:2:0) and block
+// form (half-precision CDEF taps up to 10 bits, integer ones above); a frame
+// with a plane written straight to the output takes the 256-thread body that
+// does so, whatever the threads per tile.
+template <class Block>
+static cudaError_t launch_dbcdef_as(const DbCdefArgs& a, bool direct, int threads, dim3 grid, size_t smem,
+                                    cudaStream_t stream) {
+    const int layout = a.ssx | a.ssy << 1;
+    if (direct) {
+        auto k = layout == 3   ? dbcdef_kernel<256, 4, 3, Block, true>
+                 : layout == 1 ? dbcdef_kernel<256, 4, 1, Block, true>
+                               : dbcdef_kernel<256, 4, 0, Block, true>;
+        return launch_overlapped(k, grid, dim3(256), smem, stream, a);
+    }
+    if (threads == 128) {
+        auto k = layout == 3   ? dbcdef_kernel<128, 5, 3, Block>
+                 : layout == 1 ? dbcdef_kernel<128, 5, 1, Block>
+                               : dbcdef_kernel<128, 5, 0, Block>;
+        return launch_overlapped(k, grid, dim3(128), smem, stream, a);
+    }
+    auto k = layout == 3   ? dbcdef_kernel<256, 4, 3, Block>
+             : layout == 1 ? dbcdef_kernel<256, 4, 1, Block>
+                           : dbcdef_kernel<256, 4, 0, Block>;
+    return launch_overlapped(k, grid, dim3(256), smem, stream, a);
 }
 
 cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream) {
@@ -825,43 +870,39 @@ cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream) {
     const size_t smem = build_dbcdef_args(L, &a);
     cudaError_t e = dbcdef_kernel_attributes();
     if (e != cudaSuccess) return e;
-    dim3 grid(div_up(L.info.mi_cols, 16), div_up(L.info.mi_rows, 16));
-    // one kernel per chroma layout (4:4:4 and monochrome, 4:2:2, 4:2:0); a
-    // frame with a plane written straight to the output takes the 256-thread
-    // body that does so, whatever the threads per tile
-    const int layout = a.ssx | a.ssy << 1;
-    if (a.direct[0].out.data || a.direct[1].out.data || a.direct[2].out.data) {
-        auto k = layout == 3   ? dbcdef_kernel<256, 4, 3, true>
-                 : layout == 1 ? dbcdef_kernel<256, 4, 1, true>
-                               : dbcdef_kernel<256, 4, 0, true>;
-        return launch_overlapped(k, grid, dim3(256), smem, stream, a);
+    const dim3 grid(div_up(L.info.mi_cols, 16), div_up(L.info.mi_rows, 16));
+    const bool direct = a.direct[0].out.data || a.direct[1].out.data || a.direct[2].out.data;
+    return a.bit_depth <= 10 ? launch_dbcdef_as<HalfBlock>(a, direct, L.threads, grid, smem, stream)
+                             : launch_dbcdef_as<PairBlock>(a, direct, L.threads, grid, smem, stream);
+}
+
+template <class Block>
+static cudaError_t launch_dbcdef_batch_as(const DbCdefArgs* args, const int* dev_prefix, int n, int tiles, size_t smem,
+                                          int ctas_per_sm, int threads, int layout, cudaStream_t stream) {
+    using K = void (*)(const DbCdefArgs*, const int*, int);
+    K k;
+    if (threads == 128) {
+        k = dbcdef_batch_kernel<128, 5, -1, Block>;
+    } else if (ctas_per_sm <= 3) {  // up to 3 resident: the 80-register body
+        k = layout == 3 ? dbcdef_batch_kernel<256, 3, 3, Block> : layout == 1 ? dbcdef_batch_kernel<256, 3, 1, Block>
+          : layout == 0 ? dbcdef_batch_kernel<256, 3, 0, Block> : dbcdef_batch_kernel<256, 3, -1, Block>;
+    } else {  // 64 registers: the layout-specialised bodies would spill
+        k = dbcdef_batch_kernel<256, 4, -1, Block>;
     }
-    if (L.threads == 128) {
-        auto k = layout == 3 ? dbcdef_kernel<128, 5, 3> : layout == 1 ? dbcdef_kernel<128, 5, 1> : dbcdef_kernel<128, 5, 0>;
-        return launch_overlapped(k, grid, dim3(128), smem, stream, a);
-    }
-    auto k = layout == 3 ? dbcdef_kernel<256, 4, 3> : layout == 1 ? dbcdef_kernel<256, 4, 1> : dbcdef_kernel<256, 4, 0>;
-    return launch_overlapped(k, grid, dim3(256), smem, stream, a);
+    k<<<tiles, threads == 128 ? 128 : 256, smem, stream>>>(args, dev_prefix, n);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_dbcdef_batch(const void* dev_args, const int* dev_prefix, int n, int tiles, size_t smem,
-                                int ctas_per_sm, int threads, int layout, cudaStream_t stream) {
+                                int ctas_per_sm, int threads, int layout, int max_bit_depth, cudaStream_t stream) {
     if (tiles <= 0) return cudaSuccess;
     cudaError_t e = dbcdef_kernel_attributes();
     if (e != cudaSuccess) return e;
     const DbCdefArgs* args = static_cast<const DbCdefArgs*>(dev_args);
-    using K = void (*)(const DbCdefArgs*, const int*, int);
-    K k;
-    if (threads == 128) {
-        k = dbcdef_batch_kernel<128, 5, -1>;
-    } else if (ctas_per_sm <= 3) {  // up to 3 resident: the 80-register body
-        k = layout == 3 ? dbcdef_batch_kernel<256, 3, 3> : layout == 1 ? dbcdef_batch_kernel<256, 3, 1>
-          : layout == 0 ? dbcdef_batch_kernel<256, 3, 0> : dbcdef_batch_kernel<256, 3, -1>;
-    } else {  // 64 registers: the layout-specialised bodies would spill
-        k = dbcdef_batch_kernel<256, 4, -1>;
-    }
-    k<<<tiles, threads == 128 ? 128 : 256, smem, stream>>>(args, dev_prefix, n);
-    return cudaGetLastError();
+    return max_bit_depth <= 10
+               ? launch_dbcdef_batch_as<HalfBlock>(args, dev_prefix, n, tiles, smem, ctas_per_sm, threads, layout, stream)
+               : launch_dbcdef_batch_as<PairBlock>(args, dev_prefix, n, tiles, smem, ctas_per_sm, threads, layout,
+                                                   stream);
 }
 
 }  // namespace vaco
