@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kThreads) cdef_frame_kernel(CdefFrameArgs a) {
     tile[0] = smem;
     tile[1] = smem + kLumaRows * kLumaPitch;
     tile[2] = tile[1] + crows * cpitch;
-    __shared__ int s_cost[64][8];
+    __shared__ uint32_t s_cost[8][64];  // per direction and block
     __shared__ BlockFilter s_filter[3][64];
     __shared__ uint8_t s_active[64];
     __shared__ int s_bad, s_any;
@@ -145,10 +145,10 @@ __global__ void __launch_bounds__(kThreads) cdef_frame_kernel(CdefFrameArgs a) {
         const int pair = warp & 3, b = ((warp >> 2) << 5) + lane;
         if (s_active[b]) {
             const uint16_t* blk = tile[0] + (2 + (b >> 3) * 8) * kLumaPitch + 8 + (b & 7) * 8;
-            int lo, hi;
+            uint32_t lo, hi;
             dir_costs_pair(pair, blk, kLumaPitch, a.shift, lo, hi);
-            s_cost[b][pair] = lo;
-            s_cost[b][pair + 4] = hi;
+            s_cost[pair][b] = lo;
+            s_cost[pair + 4][b] = hi;
         }
     }
     __syncthreads();
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kThreads) cdef_frame_kernel(CdefFrameArgs a) {
         const int b = tid;
         int dir = 0;
         uint32_t var = 0;
-        if (a.bd_ok) best_direction(s_cost[b], dir, var);
+        if (a.bd_ok) best_direction(s_cost, b, dir, var);
         bool param_bad[3] = {false, false, false};
         for (int p = 0; p < a.num_planes; ++p) {
             bool chroma = p != 0;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kThreads) cdef_frame_kernel(CdefFrameArgs a) {
                     if (!chroma) {
                         int dir;
                         uint32_t var;
-                        best_direction(s_cost[b], dir, var);
+                        best_direction(s_cost, b, dir, var);
                         primary = adjust_strength(primary, var);
                     }
                     int damping = (a.damping + a.shift - (chroma ? 1 : 0)) & 0xFF;
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kThreads) find_direction_kernel(const uint16_t
                                                                   int bit_depth, uint8_t* dirs, uint32_t* vars,
                                                                   DeviceStatus* status) {
     __shared__ __align__(16) uint16_t sm[64 * 64];
-    __shared__ int s_cost[64][8];
+    __shared__ uint32_t s_cost[8][64];  // per direction and block
     const int base = blockIdx.x * 64;
     const int tid = threadIdx.x;
     const bool bd_ok = bit_depth == 8 || bit_depth == 10 || bit_depth == 12;
@@ -305,15 +305,15 @@ __global__ void __launch_bounds__(kThreads) find_direction_kernel(const uint16_t
     if (!bd_ok) return;
     const int warp = tid >> 5, lane = tid & 31;
     const int pair = warp & 3, b = ((warp >> 2) << 5) + lane;
-    int lo, hi;
+    uint32_t lo, hi;
     dir_costs_pair(pair, sm + b * 64, 8, bit_depth - 8, lo, hi);
-    s_cost[b][pair] = lo;
-    s_cost[b][pair + 4] = hi;
+    s_cost[pair][b] = lo;
+    s_cost[pair + 4][b] = hi;
     __syncthreads();
     if (tid < 64 && base + tid < n) {
         int d;
         uint32_t v;
-        best_direction(s_cost[tid], d, v);
+        best_direction(s_cost, tid, d, v);
         dirs[base + tid] = (uint8_t)d;
         vars[base + tid] = v;
     }

@@ -59,36 +59,86 @@ __host__ __device__ constexpr int dir_weight(int d, int b) {
     return dir_count(d, b) ? 840 / dir_count(d, b) : 0;
 }
 
-// Costs of directions P and P+4 for one 8x8 block at `blk` (row pitch in
-// samples, rows 16-byte aligned).  Fully unrolled: every bin is a register.
-template <int P>
-__device__ __forceinline__ void dir_costs(const uint16_t* blk, int pitch, int shift, int& c_lo, int& c_hi) {
-    int a[15], b[15];
+// How a direction's lines meet the words of two samples that a row is read as
+// (word k of row i: samples 2k, 2k+1).
+constexpr bool dir_word_in_one_line(int d) { return dir_bin(d, 0, 0) == dir_bin(d, 0, 1); }  // 1, 2, 3
+constexpr bool dir_row_pair(int d) { return dir_bin(d, 0, 0) == dir_bin(d, 1, 0); }          // 5, 6, 7
+
+// Sum over the lines of direction D of (line sum)^2 * 840 / (line length) for
+// the 8-bit samples of a block, two per word in w[row][word].
+//
+// vaco subtracts 128 from every sample first (src/cdef.rs:99-112).  With 840 /
+// length exact for every length (1..8), that changes each direction's cost by
+// the same amount, -256 * 840 * (sum of all) + 128^2 * 840 * 64, and only
+// differences of costs are used; left out, a cost is at most 840 * 64 * 255^2
+// < 2^32.
+//
+// Line sums are built two at a time: a word whose samples lie on two adjacent
+// lines adds to one packed accumulator (at most 8 * 255 per half).  Words that
+// start on an even line and on an odd line have accumulators of their own, so
+// no word is taken apart; a byte permute lines the two up at the end.
+template <int D>
+__device__ __forceinline__ uint32_t dir_cost(const uint32_t (&w)[8][4]) {
+    static_assert(D >= 0 && D < 8, "direction");
+    uint32_t cost = 0;
+    auto add = [&](uint32_t sum, int line) {
+        if (line >= 0 && line < 15 && dir_weight(D, line)) cost += sum * (sum * (uint32_t)dir_weight(D, line));
+    };
+    if (dir_word_in_one_line(D)) {
+        uint32_t acc[11] = {};
 #pragma unroll
-    for (int k = 0; k < 15; ++k) a[k] = b[k] = 0;
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        uint4 row = *reinterpret_cast<const uint4*>(blk + i * pitch);
-        uint32_t w[4] = {row.x, row.y, row.z, row.w};
+            for (int k = 0; k < 4; ++k) acc[dir_bin(D, i, 2 * k)] += w[i][k];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            int s = (j & 1) ? (w[j >> 1] >> 16) : (w[j >> 1] & 0xFFFF);
-            int v = (s >> shift) - 128;
-            a[dir_bin(P, i, j)] += v;
-            b[dir_bin(P + 4, i, j)] += v;
+        for (int l = 0; l < 11; ++l) add((acc[l] * 0x10001u) >> 16, l);  // both halves' sum
+        return cost;
+    }
+    // even[m] holds lines 2m, 2m+1 and odd[m + 1] lines 2m+1, 2m+2, in
+    // ascending order of samples for all but direction 4, whose lines descend
+    // along a row (the halves then swap roles).
+    constexpr bool down = dir_bin(D, 0, 1) < dir_bin(D, 0, 0);
+    constexpr int step = dir_row_pair(D) ? 2 : 1;
+    uint32_t even[8] = {}, odd[9] = {};
+#pragma unroll
+    for (int i = 0; i < 8; i += step)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t v = step == 2 ? w[i][k] + w[i + (step - 1)][k] : w[i][k];
+            const int low = down ? dir_bin(D, i, 2 * k + 1) : dir_bin(D, i, 2 * k);  // lower line of the two
+            if ((low & 1) == 0) even[low >> 1] += v;
+            else odd[(low + 1) >> 1] += v;
         }
-    }
-    int lo = 0, hi = 0;
 #pragma unroll
-    for (int k = 0; k < 15; ++k) {
-        if (dir_weight(P, k)) lo += a[k] * a[k] * dir_weight(P, k);
-        if (dir_weight(P + 4, k)) hi += b[k] * b[k] * dir_weight(P + 4, k);
+    for (int m = 0; m < 8; ++m) {
+        // odd[m]: lines 2m-1 and 2m; odd[m + 1]: lines 2m+1 and 2m+2
+        const uint32_t x = even[m] + (down ? __byte_perm(odd[m + 1], odd[m], 0x5432)
+                                           : __byte_perm(odd[m], odd[m + 1], 0x5432));
+        add(down ? x >> 16 : x & 0xFFFFu, 2 * m);
+        add(down ? x & 0xFFFFu : x >> 16, 2 * m + 1);
     }
-    c_lo = lo;
-    c_hi = hi;
+    return cost;
 }
 
-__device__ __forceinline__ void dir_costs_pair(int pair, const uint16_t* blk, int pitch, int shift, int& lo, int& hi) {
+// Costs of directions P and P+4 for one 8x8 block at `blk` (row pitch in
+// samples, rows 16-byte aligned), samples scaled to 8 bits.  Fully unrolled.
+template <int P>
+__device__ __forceinline__ void dir_costs(const uint16_t* blk, int pitch, int shift, uint32_t& lo, uint32_t& hi) {
+    uint32_t w[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint4 row = *reinterpret_cast<const uint4*>(blk + i * pitch);
+        w[i][0] = (row.x >> shift) & 0x00FF00FFu;
+        w[i][1] = (row.y >> shift) & 0x00FF00FFu;
+        w[i][2] = (row.z >> shift) & 0x00FF00FFu;
+        w[i][3] = (row.w >> shift) & 0x00FF00FFu;
+    }
+    lo = dir_cost<P>(w);
+    hi = dir_cost<P + 4>(w);
+}
+
+__device__ __forceinline__ void dir_costs_pair(int pair, const uint16_t* blk, int pitch, int shift, uint32_t& lo,
+                                               uint32_t& hi) {
     switch (pair) {
         case 0: dir_costs<0>(blk, pitch, shift, lo, hi); break;
         case 1: dir_costs<1>(blk, pitch, shift, lo, hi); break;
@@ -97,13 +147,20 @@ __device__ __forceinline__ void dir_costs_pair(int pair, const uint16_t* blk, in
     }
 }
 
-__device__ __forceinline__ void best_direction(const int* cost8, int& best, uint32_t& var) {
-    int b = 0;
+// The first direction of the largest cost; cost[d][b] for block b.
+__device__ __forceinline__ void best_direction(const uint32_t (*cost)[64], int b, int& best, uint32_t& var) {
+    int bd = 0;
+    uint32_t top = cost[0][b];
 #pragma unroll
-    for (int d = 1; d < 8; ++d)
-        if (cost8[d] > cost8[b]) b = d;
-    best = b;
-    var = (uint32_t)((cost8[b] - cost8[(b + 4) & 7]) >> 10);
+    for (int d = 1; d < 8; ++d) {
+        const uint32_t c = cost[d][b];
+        if (c > top) {
+            top = c;
+            bd = d;
+        }
+    }
+    best = bd;
+    var = (top - cost[(bd + 4) & 7][b]) >> 10;
 }
 
 // constrain (src/cdef.rs:126-133); threshold 0 yields 0 for any shift.

@@ -416,7 +416,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     // (every plane geometry below becomes a constant); LAYOUT < 0 reads it
     const int ssx = LAYOUT < 0 ? a.ssx : (LAYOUT & 1), ssy = LAYOUT < 0 ? a.ssy : (LAYOUT >> 1);
     extern __shared__ __align__(16) uint16_t smem[];
-    __shared__ int s_cost[64][8];
+    __shared__ uint32_t s_cost[8][64];  // per direction and block
     __shared__ Block s_block[2][64];  // luma, chroma (U and V share strengths and directions)
     __shared__ uint8_t s_active[64];
     __shared__ int s_count[8];  // list lengths per size class, pass 0 then pass 1
@@ -647,10 +647,10 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         const int pair = job & 3, b = ((job >> 2) << 5) + lane;
         if (s_active[b]) {
             const uint16_t* blk = smem + a.plane_off[0] + (kHalo + (b >> 3) * 8) * lpitch + kHalo + (b & 7) * 8;
-            int lo, hi;
+            uint32_t lo, hi;
             dir_costs_pair(pair, blk, lpitch, a.shift, lo, hi);
-            s_cost[b][pair] = lo;
-            s_cost[b][pair + 4] = hi;
+            s_cost[pair][b] = lo;
+            s_cost[pair + 4][b] = hi;
         }
     }
     __syncthreads();
@@ -661,7 +661,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         const bool chroma = i >= 64;
         int dir;
         uint32_t var;
-        best_direction(s_cost[b], dir, var);
+        best_direction(s_cost, b, dir, var);
         int sp = 0, ss = 0;
         if (index < 8) {
             sp = chroma ? a.uv_pri[index] : a.y_pri[index];
