@@ -232,23 +232,11 @@ __device__ __forceinline__ void shift_copy(const uint16_t* t, uint32_t* shifted)
     }
 }
 
-// Segment-list entry: level (6 bits) | samples on the q side, capped at 8 (4)
-// | on the p side, capped at 8 (4) | staged offset of q0 on the segment's
+// Segment-list entry: level (6 bits) | staged offset of q0 on the segment's
 // first line (13) | plane (2) | first cell of its edge (1) | last cell (1).
-// Capping at 8 keeps the clamping of load_line / store_at exact: no filter
-// reaches more than 7 samples from its edge.
-__device__ __forceinline__ uint32_t seg_entry(int lvl, int nq, int np, int off, int p, bool first, bool last) {
-    return (uint32_t)lvl | ((uint32_t)min(nq, 8) << 6) | ((uint32_t)min(np, 8) << 10) | ((uint32_t)off << 14) |
-           ((uint32_t)p << 27) | ((uint32_t)first << 29) | ((uint32_t)last << 30);
-}
-
-template <int STEP>
-__device__ __forceinline__ void filter_line_class(int cls, uint16_t* q, int step, int nq, int np, const Strength& s,
-                                                  int bd) {
-    if (cls == 0) line_size4<STEP>(q, step, nq, np, s, bd);
-    else if (cls == 1) line_size6<STEP>(q, step, nq, np, s, bd);
-    else if (cls == 2) line_size8<STEP>(q, step, nq, np, s, bd);
-    else line_size16<STEP>(q, step, nq, np, s, bd);
+__device__ __forceinline__ uint32_t seg_entry(int lvl, int off, int p, bool first, bool last) {
+    return (uint32_t)lvl | ((uint32_t)off << 6) | ((uint32_t)p << 19) | ((uint32_t)first << 21) |
+           ((uint32_t)last << 22);
 }
 
 // The edge segments of both deblocking passes over the staged tiles of every
@@ -320,7 +308,7 @@ __device__ __forceinline__ void deblock_lists(const DbCdefArgs& a, int ssx, int 
                     const int size = min(p ? 8 : 16, 1 << min(cl, pl));
                     const int cls = size == 4 ? 0 : p ? 1 : size == 8 ? 2 : 3;
                     const int at = atomicAdd(&s_count[cls], 1);
-                    s_list[c_list_off[cls] + at] = seg_entry(lvl, P.width - xp, xp, off, p, cr == 0, cr == nr - 1);
+                    s_list[c_list_off[cls] + at] = seg_entry(lvl, off, p, cr == 0, cr == nr - 1);
                 }
             }
         }
@@ -339,8 +327,7 @@ __device__ __forceinline__ void deblock_lists(const DbCdefArgs& a, int ssx, int 
                     const int size = min(p ? 8 : 16, 1 << min(cl, pl));
                     const int cls = size == 4 ? 0 : p ? 1 : size == 8 ? 2 : 3;
                     const int at = atomicAdd(&s_count[4 + cls], 1);
-                    s_list[kListTotal + c_list_off[cls] + at] =
-                        seg_entry(lvl, P.height - yp, yp, off, p, cc == 0, cc == ncol - 1);
+                    s_list[kListTotal + c_list_off[cls] + at] = seg_entry(lvl, off, p, cc == 0, cc == ncol - 1);
                 }
             }
         }
@@ -353,6 +340,15 @@ __device__ __forceinline__ void deblock_lists(const DbCdefArgs& a, int ssx, int 
 // rows [py0-7, py0+th+7) / [py0-3, py0+th+3) in pass 0, columns [px0-2,
 // px0+tw+2) in pass 1.  Within a pass no two edges touch a common sample, so
 // the lines run in place in any order.
+//
+// No filter reaches past the plane: an edge of filter size n sits on a
+// multiple of n (it is a transform edge of a transform at least n wide) and
+// not on 0, so n samples lie before it; and the planes are Mi-padded (luma
+// extents multiples of 8, chroma of 4), which leaves at least 8 samples after
+// an edge of luma size 8 or 16 and 4 after any other, against reaches of 4, 7
+// and, for chroma and size 4, 3.  So there are no clamped reads.  (A second,
+// clamping body per class made the kernel 110 KB of code instead of 79 KB and
+// a 4K 10-bit frame 1.2 % slower, without ever running.)
 template <int PASS, int NT>
 __device__ __forceinline__ void deblock_filter(const DbCdefArgs& a, int ssx, int ssy, uint16_t* smem,
                                                const uint32_t* s_list, const int* s_count,
@@ -383,25 +379,12 @@ __device__ __forceinline__ void deblock_filter(const DbCdefArgs& a, int ssx, int
             }
         }
         const uint32_t e = s_list[c_list_off[cls] + seg];
-        const bool first = (e >> 29) & 1, last = (e >> 30) & 1;
+        const bool first = (e >> 21) & 1, last = (e >> 22) & 1;
         if (PASS == 1 && ((first && h == 0) || (last && h == 1))) continue;
-        const int lvl = e & 63, nq = (e >> 6) & 15, np = (e >> 10) & 15, off = (e >> 14) & 0x1FFF, p = (e >> 27) & 3;
+        const int lvl = e & 63, off = (e >> 6) & 0x1FFF, p = (e >> 19) & 3;
         const int pitch = p ? gc.pitch : gl.pitch;
         uint16_t* q = smem + a.plane_off[p] + off + (PASS == 0 ? 2 * h * pitch : 2 * h);
-        const int reach = class_reach(cls);
-        if (nq >= reach && np >= reach) {
-            filter_pair_class<PASS>(cls, q, pitch, s_str[lvl], a.bit_depth - 8);
-        } else {
-            // near the plane edge: line by line, with clamped reads and
-            // dropped writes
-            const Strength s = strength_of(lvl, a.sharpness);
-            for (int l = 0; l < 2; ++l) {
-                if (PASS == 0)
-                    filter_line_class<1>(cls, q + l * pitch, 1, nq, np, s, a.bit_depth);
-                else
-                    filter_line_class<0>(cls, q + l, pitch, nq, np, s, a.bit_depth);
-            }
-        }
+        filter_pair_class<PASS>(cls, q, pitch, s_str[lvl], a.bit_depth - 8);
     }
     __syncthreads();
 }

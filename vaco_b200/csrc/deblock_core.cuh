@@ -131,175 +131,10 @@ __device__ __forceinline__ int level_at(const DeblockLaunch& L, int plane, int p
 namespace vaco {
 namespace dbk {
 
-// ---------------------------------------------------------------- size-class line filters
-//
-// The same arithmetic as filter_line(), split by filter size so that a warp
-// runs one class at a time.  q points at q0; sample k of the line (k < 0 is
-// the p side) lives at q[k * step].  nq / np count the samples that exist on
-// each side inside the plane: when both reach past the filter's span the
-// loads need no clamping, otherwise reads repeat the last sample and writes
-// past the plane are dropped (the get_clamped / set semantics of the oracle).
-
-template <int R, int STEP>
-__device__ __forceinline__ void load_line(const uint16_t* q, long step_rt, int nq, int np, int* Pv, int* Qv) {
-    const long step = STEP ? STEP : step_rt;
-    if (nq >= R && np >= R) {
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            Qv[k] = q[k * step];
-            Pv[k] = q[-(k + 1) * step];
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            Qv[k] = q[min(k, nq - 1) * step];
-            Pv[k] = q[-min(k + 1, np) * step];
-        }
-    }
-}
-
-template <int STEP>
-__device__ __forceinline__ void store_at(uint16_t* q, long step_rt, int nq, int np, int k, int v) {
-    const long step = STEP ? STEP : step_rt;
-    if (k >= 0 ? k < nq : -k <= np) q[k * step] = (uint16_t)v;
-}
-
-// 7.14.6.3 narrow filter on p1, p0, q0, q1.
-template <int STEP>
-__device__ __forceinline__ void narrow_apply(uint16_t* q, long step_rt, int nq, int np, int p1, int p0, int q0, int q1,
-                                             bool hev, int bd) {
-    const int sh = bd - 8, half = 0x80 << sh, lo = -(1 << (bd - 1)), hi = (1 << (bd - 1)) - 1;
-    const int ps1 = p1 - half, ps0 = p0 - half, qs0 = q0 - half, qs1 = q1 - half;
-    int f = hev ? clampi(ps1 - qs1, lo, hi) : 0;
-    f = clampi(f + 3 * (qs0 - ps0), lo, hi);
-    const int f1 = clampi(f + 4, lo, hi) >> 3;
-    const int f2 = clampi(f + 3, lo, hi) >> 3;
-    store_at<STEP>(q, step_rt, nq, np, 0, clampi(qs0 - f1, lo, hi) + half);
-    store_at<STEP>(q, step_rt, nq, np, -1, clampi(ps0 + f2, lo, hi) + half);
-    if (!hev) {
-        const int f3 = (f1 + 1) >> 1;
-        store_at<STEP>(q, step_rt, nq, np, 1, clampi(qs1 - f3, lo, hi) + half);
-        store_at<STEP>(q, step_rt, nq, np, -2, clampi(ps1 + f3, lo, hi) + half);
-    }
-}
-
-// Filter size 4 (luma or chroma): mask over p1..q1, narrow filter.
-template <int STEP>
-__device__ __forceinline__ void line_size4(uint16_t* q, long step_rt, int nq, int np, const Strength& s, int bd) {
-    int P[2], Q[2];
-    load_line<2, STEP>(q, step_rt, nq, np, P, Q);
-    const int sh = bd - 8;
-    const int limit = s.limit << sh, blimit = s.blimit << sh, thresh = s.thresh << sh;
-    const int d_p = abs(P[1] - P[0]), d_q = abs(Q[1] - Q[0]);
-    if (max(d_p, d_q) > limit || abs(P[0] - Q[0]) * 2 + abs(P[1] - Q[1]) / 2 > blimit) return;
-    narrow_apply<STEP>(q, step_rt, nq, np, P[1], P[0], Q[0], Q[1], max(d_p, d_q) > thresh, bd);
-}
-
-// Filter size 8 on a chroma plane (filter length 6).
-template <int STEP>
-__device__ __forceinline__ void line_size6(uint16_t* q, long step_rt, int nq, int np, const Strength& s, int bd) {
-    int P[3], Q[3];
-    load_line<3, STEP>(q, step_rt, nq, np, P, Q);
-    const int sh = bd - 8;
-    const int limit = s.limit << sh, blimit = s.blimit << sh, thresh = s.thresh << sh;
-    const int d_p = abs(P[1] - P[0]), d_q = abs(Q[1] - Q[0]);
-    const int m = max(max(d_p, d_q), max(abs(P[2] - P[1]), abs(Q[2] - Q[1])));
-    if (m > limit || abs(P[0] - Q[0]) * 2 + abs(P[1] - Q[1]) / 2 > blimit) return;
-    const int one = 1 << sh;
-    const bool flat = max(max(d_p, d_q), max(abs(P[2] - P[0]), abs(Q[2] - Q[0]))) <= one;
-    if (!flat) {
-        narrow_apply<STEP>(q, step_rt, nq, np, P[1], P[0], Q[0], Q[1], max(d_p, d_q) > thresh, bd);
-        return;
-    }
-    const int p2 = P[2], p1 = P[1], p0 = P[0], q0 = Q[0], q1 = Q[1], q2 = Q[2];
-    store_at<STEP>(q, step_rt, nq, np, -2, (3 * p2 + 2 * p1 + 2 * p0 + q0 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, -1, (p2 + 2 * p1 + 2 * p0 + 2 * q0 + q1 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, 0, (p1 + 2 * p0 + 2 * q0 + 2 * q1 + q2 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, 1, (p0 + 2 * q0 + 2 * q1 + 3 * q2 + 4) >> 3);
-}
-
-template <int STEP>
-__device__ __forceinline__ void apply8(uint16_t* q, long step_rt, int nq, int np, const int* P, const int* Q) {
-    const int p3 = P[3], p2 = P[2], p1 = P[1], p0 = P[0], q0 = Q[0], q1 = Q[1], q2 = Q[2], q3 = Q[3];
-    store_at<STEP>(q, step_rt, nq, np, -3, (3 * p3 + 2 * p2 + p1 + p0 + q0 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, -2, (2 * p3 + p2 + 2 * p1 + p0 + q0 + q1 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, -1, (p3 + p2 + p1 + 2 * p0 + q0 + q1 + q2 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, 0, (p2 + p1 + p0 + 2 * q0 + q1 + q2 + q3 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, 1, (p1 + p0 + q0 + 2 * q1 + q2 + 2 * q3 + 4) >> 3);
-    store_at<STEP>(q, step_rt, nq, np, 2, (p0 + q0 + q1 + 2 * q2 + 3 * q3 + 4) >> 3);
-}
-
-// Filter size 8 on luma (filter length 8).
-template <int STEP>
-__device__ __forceinline__ void line_size8(uint16_t* q, long step_rt, int nq, int np, const Strength& s, int bd) {
-    int P[4], Q[4];
-    load_line<4, STEP>(q, step_rt, nq, np, P, Q);
-    const int sh = bd - 8;
-    const int limit = s.limit << sh, blimit = s.blimit << sh, thresh = s.thresh << sh;
-    const int d_p = abs(P[1] - P[0]), d_q = abs(Q[1] - Q[0]);
-    const int m = max(max(max(d_p, d_q), max(abs(P[2] - P[1]), abs(Q[2] - Q[1]))),
-                      max(abs(P[3] - P[2]), abs(Q[3] - Q[2])));
-    if (m > limit || abs(P[0] - Q[0]) * 2 + abs(P[1] - Q[1]) / 2 > blimit) return;
-    const int one = 1 << sh;
-    const int fl = max(max(max(d_p, d_q), max(abs(P[2] - P[0]), abs(Q[2] - Q[0]))),
-                       max(abs(P[3] - P[0]), abs(Q[3] - Q[0])));
-    if (fl > one) {
-        narrow_apply<STEP>(q, step_rt, nq, np, P[1], P[0], Q[0], Q[1], max(d_p, d_q) > thresh, bd);
-        return;
-    }
-    apply8<STEP>(q, step_rt, nq, np, P, Q);
-}
-
-// Filter size 16 on luma: narrow, 8-tap or 14-tap by the flat masks.
-template <int STEP>
-__device__ __forceinline__ void line_size16(uint16_t* q, long step_rt, int nq, int np, const Strength& s, int bd) {
-    int P[7], Q[7];
-    load_line<7, STEP>(q, step_rt, nq, np, P, Q);
-    const int sh = bd - 8;
-    const int limit = s.limit << sh, blimit = s.blimit << sh, thresh = s.thresh << sh;
-    const int d_p = abs(P[1] - P[0]), d_q = abs(Q[1] - Q[0]);
-    const int m = max(max(max(d_p, d_q), max(abs(P[2] - P[1]), abs(Q[2] - Q[1]))),
-                      max(abs(P[3] - P[2]), abs(Q[3] - Q[2])));
-    if (m > limit || abs(P[0] - Q[0]) * 2 + abs(P[1] - Q[1]) / 2 > blimit) return;
-    const int one = 1 << sh;
-    const int fl = max(max(max(d_p, d_q), max(abs(P[2] - P[0]), abs(Q[2] - Q[0]))),
-                       max(abs(P[3] - P[0]), abs(Q[3] - Q[0])));
-    if (fl > one) {
-        narrow_apply<STEP>(q, step_rt, nq, np, P[1], P[0], Q[0], Q[1], max(d_p, d_q) > thresh, bd);
-        return;
-    }
-    const int fl2 = max(max(max(abs(P[6] - P[0]), abs(Q[6] - Q[0])), max(abs(P[5] - P[0]), abs(Q[5] - Q[0]))),
-                        max(abs(P[4] - P[0]), abs(Q[4] - Q[0])));
-    if (fl2 > one) {
-        apply8<STEP>(q, step_rt, nq, np, P, Q);
-        return;
-    }
-    // 14-tap (7.14.6.4, log2Size 4): out[i] = Round2(T_i + U_i, 4) with
-    // T_i the 13-sample window sum (edge-clamped) and U_i = F[i-1]+F[i]+F[i+1].
-    int F[14];
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-        F[6 - k] = P[k];
-        F[7 + k] = Q[k];
-    }
-    int T = 6 * F[0];
-#pragma unroll
-    for (int k = 1; k <= 7; ++k) T += F[k];  // window of i = -6: F[0]x7 .. F[7]
-    int out[12];
-#pragma unroll
-    for (int i = -6; i < 6; ++i) {
-        const int c = i + 7;  // F index of output i
-        out[i + 6] = (T + F[c - 1] + F[c] + F[c + 1] + 8) >> 4;
-        if (i < 5) T += F[min(c + 7, 13)] - F[max(c - 6, 0)];
-    }
-#pragma unroll
-    for (int i = -6; i < 6; ++i) store_at<STEP>(q, step_rt, nq, np, i, out[i + 6]);
-}
-
 // ---------------------------------------------------------------- two lines per register
 //
-// The size-class filters above for two adjacent lines of one edge segment at
-// once: sample k of both lines sits in one 32-bit word, the first line in the
+// The arithmetic of filter_line(), split by filter size so that a warp runs one
+// class at a time, for two adjacent lines of one edge segment at once: sample k of both lines sits in one 32-bit word, the first line in the
 // low 16 bits.  Both lines share the segment's filter size and strengths;
 // each keeps its own masks (filterMask, hev, flat, flat2 of 7.14.6.2), which
 // select per 16-bit half between the original samples and the narrow, 8-tap
@@ -313,9 +148,8 @@ __device__ __forceinline__ void line_size16(uint16_t* q, long step_rt, int nq, i
 //     take (|ps1 - qs1| + 3 |qs0 - ps0| <= 4 x 4095), and whose multiples of
 //     8 and 16 keep the arithmetic shifts exact: (v + 2^14) >> 3 =
 //     (v >> 3) + 2^11 for any v > -2^14.
-// The callers use these only where the segment reaches R samples into the
-// plane on both sides (no clamped reads, no dropped writes); nearer the plane
-// edge they run the per-line filters above.
+// The fused kernel's planes leave every filter its full reach on both sides of
+// an edge (see deblock_filter()), so no read is clamped and no write dropped.
 
 __device__ __forceinline__ uint32_t pmin2(uint32_t a, uint32_t b) {
     uint32_t d;
@@ -435,7 +269,7 @@ __device__ __forceinline__ void store_pair(uint16_t* q, int pitch, const uint32_
     }
 }
 
-// The 8-tap outputs (samples -3 .. 2) of apply8 into w[0..5].
+// The 8-tap outputs (samples -3 .. 2) into w[0..5].
 __device__ __forceinline__ void wide8_2(const uint32_t* P, const uint32_t* Q, uint32_t* w) {
     const uint32_t p3 = P[3], p2 = P[2], p1 = P[1], p0 = P[0], q0 = Q[0], q1 = Q[1], q2 = Q[2], q3 = Q[3];
     const uint32_t r = pk2(4), m = 0x1FFF1FFFu;
@@ -579,7 +413,7 @@ __device__ __forceinline__ void pair_size16(uint16_t* q, int pitch, const PairSt
     for (int k = 0; k < 4; ++k) o[4 + k] = sel2(narrow, n[k], o[4 + k]);
     if (flat2 != 0) {
         // 14-tap (log2Size 4): out[i] = (T_i + F[i-1] + F[i] + F[i+1] + 8) >> 4
-        // with T_i the edge-clamped 13-sample window sum, as line_size16
+        // with T_i the edge-clamped 13-sample window sum
         uint32_t F[14];
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
@@ -618,10 +452,6 @@ __device__ __forceinline__ void filter_pair_class(int cls, uint16_t* q, int pitc
     else if (cls == 2) pair_size8<PASS>(q, pitch, s, sh);
     else pair_size16<PASS>(q, pitch, s, sh);
 }
-
-// Samples per side a size class reads (and the per-line filters' clamping
-// threshold): 4-tap 2, chroma 6-tap 3, luma 8-tap 4, luma 14-tap 7.
-__device__ __forceinline__ int class_reach(int cls) { return cls == 0 ? 2 : cls == 1 ? 3 : cls == 2 ? 4 : 7; }
 
 }  // namespace dbk
 }  // namespace vaco
