@@ -922,6 +922,7 @@ static int32_t postfilter_dev_impl(vaco_av1_ctx* ctx, cudaStream_t s, const vaco
             L.cdef = cp;
             L.status = ctx->status;
             L.threads = ctx->tuning.dbcdef_threads == 128 ? 128 : 256;
+            L.sm_count = ctx->sm_count;
             for (int k = 0; k < 3; ++k) L.direct[k] = direct[k];
             e = launch_dbcdef(L, s);
             ctx->launches++;

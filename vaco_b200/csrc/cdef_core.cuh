@@ -120,11 +120,9 @@ __device__ __forceinline__ uint32_t dir_cost(const uint32_t (&w)[8][4]) {
     return cost;
 }
 
-// Costs of directions P and P+4 for one 8x8 block at `blk` (row pitch in
-// samples, rows 16-byte aligned), samples scaled to 8 bits.  Fully unrolled.
-template <int P>
-__device__ __forceinline__ void dir_costs(const uint16_t* blk, int pitch, int shift, uint32_t& lo, uint32_t& hi) {
-    uint32_t w[8][4];
+// The words of an 8x8 block at `blk` (row pitch in samples, rows 16-byte
+// aligned), samples scaled to 8 bits.
+__device__ __forceinline__ void dir_load(const uint16_t* blk, int pitch, int shift, uint32_t (&w)[8][4]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const uint4 row = *reinterpret_cast<const uint4*>(blk + i * pitch);
@@ -133,6 +131,14 @@ __device__ __forceinline__ void dir_costs(const uint16_t* blk, int pitch, int sh
         w[i][2] = (row.z >> shift) & 0x00FF00FFu;
         w[i][3] = (row.w >> shift) & 0x00FF00FFu;
     }
+}
+
+// Costs of directions pair and pair + 4, or of direction d alone.  Fully
+// unrolled per direction; the switches are warp-uniform.
+template <int P>
+__device__ __forceinline__ void dir_costs(const uint16_t* blk, int pitch, int shift, uint32_t& lo, uint32_t& hi) {
+    uint32_t w[8][4];
+    dir_load(blk, pitch, shift, w);
     lo = dir_cost<P>(w);
     hi = dir_cost<P + 4>(w);
 }
@@ -144,6 +150,21 @@ __device__ __forceinline__ void dir_costs_pair(int pair, const uint16_t* blk, in
         case 1: dir_costs<1>(blk, pitch, shift, lo, hi); break;
         case 2: dir_costs<2>(blk, pitch, shift, lo, hi); break;
         default: dir_costs<3>(blk, pitch, shift, lo, hi); break;
+    }
+}
+
+__device__ __forceinline__ uint32_t dir_cost_of(int d, const uint16_t* blk, int pitch, int shift) {
+    uint32_t w[8][4];
+    dir_load(blk, pitch, shift, w);
+    switch (d) {
+        case 0: return dir_cost<0>(w);
+        case 1: return dir_cost<1>(w);
+        case 2: return dir_cost<2>(w);
+        case 3: return dir_cost<3>(w);
+        case 4: return dir_cost<4>(w);
+        case 5: return dir_cost<5>(w);
+        case 6: return dir_cost<6>(w);
+        default: return dir_cost<7>(w);
     }
 }
 

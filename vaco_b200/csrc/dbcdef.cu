@@ -140,12 +140,19 @@ struct PairTaps {
 // non-zero; with neither, every sample stays as it is.
 // SHIFT: the pairs that start on odd samples are at s1, rows from row kHalo-2
 // on the staged pitch, planes at the same distance.
-template <int PITCH, int BH, int RPI, int NPL, bool SHIFT, bool DIRECT, class Block>
+// PARTS warps share the block row, by plane first, then by rows; `part` is
+// this warp's share.
+template <int PITCH, int BH, int RPI, int NPL, int PARTS, bool SHIFT, bool DIRECT, class Block>
 __device__ __forceinline__ void filter_block_row(const DbCdefArgs& a, int p0, const uint16_t* t, const uint32_t* s1,
                                                  int plane_words, int px0, int py0, const uint8_t* active,
-                                                 const Block* blocks, bool pri_on, bool sec_on, int br, int lane,
-                                                 int sx) {
+                                                 const Block* blocks, bool pri_on, bool sec_on, int br, int part,
+                                                 int lane, int sx) {
     constexpr int ppr = 32 / RPI;          // pairs per row: the tile is 2 ppr samples wide
+    constexpr bool by_plane = PARTS >= NPL;
+    constexpr int row_parts = by_plane ? PARTS / NPL : 1, steps = BH / RPI / row_parts;
+    static_assert(steps >= 1, "every warp has a row");
+    const int pl0 = by_plane ? part % NPL : 0, pl1 = by_plane ? pl0 + 1 : NPL;
+    const int j0 = by_plane ? part / NPL * steps : 0;
     const int x = 2 * (lane % ppr), lr = lane / ppr;
     const int r0 = br * BH;
     const int gx = px0 + x;
@@ -160,7 +167,7 @@ __device__ __forceinline__ void filter_block_row(const DbCdefArgs& a, int p0, co
     // Runs out(word offset, value) over the lane's rows of every plane.
     auto rows = [&](auto&& value) {
 #pragma unroll 1  // smaller code: the fused kernel is sensitive to instruction fetch
-        for (int pl = 0; pl < NPL; ++pl) {
+        for (int pl = pl0; pl < pl1; ++pl) {
             const DevPlane& d = a.dst[p0 + pl];
             uint32_t* o = reinterpret_cast<uint32_t*>(d.data + (long)(py0 + r0 + lr) * d.stride + gx);
             const long ostride = (long)d.stride * RPI / 2;  // words per RPI rows
@@ -177,7 +184,7 @@ __device__ __forceinline__ void filter_block_row(const DbCdefArgs& a, int p0, co
                 }
             }
 #pragma unroll 1
-            for (int j = 0; j < BH / RPI; ++j) {
+            for (int j = j0; j < j0 + steps; ++j) {
                 const uint32_t v = value(pl * plane_words + j * (RPI * PITCH / 2));
                 if (col_in && lr + RPI * j < rows_here) o[j * ostride] = v;
                 if (DIRECT && od && lr + RPI * j < od_rows) {
@@ -623,17 +630,24 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         shift_copy<32 + 2 * kHalo, 32 + 4, NT>(smem + a.plane_off[2], sc + (32 + 2 * kHalo) * (32 + 2 * kHalo) / 2);
     }
 
-    // Direction search: job j (0..7, spread over the warps) handles direction
-    // pair (j & 3) for blocks (j >> 2)*32 + lane (warp-uniform branches).
+    // Direction search: a warp takes 32 blocks, one per lane, and a direction
+    // pair (d, d + 4), or with 16 warps and more one direction, so every
+    // branch below is warp-uniform.
     const int lpitch = 64 + 2 * kHalo;
-    for (int job = warp; job < 8; job += kWarpsNT) {
-        const int pair = job & 3, b = ((job >> 2) << 5) + lane;
+    constexpr int kDirJobs = kWarpsNT > 8 ? 16 : 8;
+    for (int job = warp; job < kDirJobs; job += kWarpsNT) {
+        const int pair = job & 3, b = (((job >> 2) & 1) << 5) + lane;
         if (s_active[b]) {
             const uint16_t* blk = smem + a.plane_off[0] + (kHalo + (b >> 3) * 8) * lpitch + kHalo + (b & 7) * 8;
-            uint32_t lo, hi;
-            dir_costs_pair(pair, blk, lpitch, a.shift, lo, hi);
-            s_cost[pair][b] = lo;
-            s_cost[pair + 4][b] = hi;
+            if (kDirJobs == 16) {
+                const int d = pair + ((job >> 3) << 2);
+                s_cost[d][b] = dir_cost_of(d, blk, lpitch, a.shift);
+            } else {
+                uint32_t lo, hi;
+                dir_costs_pair(pair, blk, lpitch, a.shift, lo, hi);
+                s_cost[pair][b] = lo;
+                s_cost[pair + 4][b] = hi;
+            }
         }
     }
     __syncthreads();
@@ -672,28 +686,32 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     // block row, lanes across the tile width; luma, then both chroma planes.
     // Tap sets of the tile's preset (uniform over the tile).
     const bool y_pri_on = index >= 8 || a.y_pri[index] != 0, y_sec_on = index >= 8 || a.y_sec[index] != 0;
-    for (int br = warp; br < 8; br += kWarpsNT)
-        filter_block_row<64 + 2 * kHalo, 8, 1, 1, true, DIRECT>(a, 0, smem + a.plane_off[0], s_u.shifted, 0, x0, y0,
-                                                                s_active, s_block[0], y_pri_on, y_sec_on, br, lane, 0);
+    constexpr int kParts = kWarpsNT > 8 ? kWarpsNT / 8 : 1;  // warps per block row
+    const int row0 = warp / kParts, part = warp % kParts;
+    constexpr int kRowStep = kWarpsNT / kParts;
+    for (int br = row0; br < 8; br += kRowStep)
+        filter_block_row<64 + 2 * kHalo, 8, 1, 1, kParts, true, DIRECT>(a, 0, smem + a.plane_off[0], s_u.shifted, 0,
+                                                                        x0, y0, s_active, s_block[0], y_pri_on,
+                                                                        y_sec_on, br, part, lane, 0);
     if (a.num_planes > 1) {
         const bool c_pri_on = index >= 8 || a.uv_pri[index] != 0, c_sec_on = index >= 8 || a.uv_sec[index] != 0;
         const uint16_t* tc = smem + a.plane_off[1];
         const int plane_words = (int)(a.plane_off[2] - a.plane_off[1]) / 2;
         const int px0 = x0 >> ssx, py0 = y0 >> ssy;
         // tile layouts: 64x64 (4:4:4), 32x32 (4:2:0), 32x64 (4:2:2)
-        for (int br = warp; br < 8; br += kWarpsNT) {
+        for (int br = row0; br < 8; br += kRowStep) {
             if (ssx == 0)
-                filter_block_row<64 + 2 * kHalo, 8, 1, 2, false, DIRECT>(a, 1, tc, nullptr, plane_words, px0, py0,
-                                                                         s_active, s_block[1], c_pri_on, c_sec_on, br,
-                                                                         lane, ssx);
+                filter_block_row<64 + 2 * kHalo, 8, 1, 2, kParts, false, DIRECT>(
+                    a, 1, tc, nullptr, plane_words, px0, py0, s_active, s_block[1], c_pri_on, c_sec_on, br, part, lane,
+                    ssx);
             else if (ssy == 1)
-                filter_block_row<32 + 2 * kHalo, 4, 2, 2, kShiftChroma, DIRECT>(
+                filter_block_row<32 + 2 * kHalo, 4, 2, 2, kParts, kShiftChroma, DIRECT>(
                     a, 1, tc, s_u.shifted + kShiftRows * (64 + 2 * kHalo) / 2, plane_words, px0, py0, s_active,
-                    s_block[1], c_pri_on, c_sec_on, br, lane, ssx);
+                    s_block[1], c_pri_on, c_sec_on, br, part, lane, ssx);
             else
-                filter_block_row<32 + 2 * kHalo, 8, 2, 2, false, DIRECT>(a, 1, tc, nullptr, plane_words, px0, py0,
-                                                                         s_active, s_block[1], c_pri_on, c_sec_on, br,
-                                                                         lane, ssx);
+                filter_block_row<32 + 2 * kHalo, 8, 2, 2, kParts, false, DIRECT>(
+                    a, 1, tc, nullptr, plane_words, px0, py0, s_active, s_block[1], c_pri_on, c_sec_on, br, part, lane,
+                    ssx);
         }
     }
 }
@@ -807,7 +825,9 @@ cudaError_t dbcdef_kernel_attributes() {
             for (auto k : {dbcdef_kernel<256, 4, 0, B>, dbcdef_kernel<256, 4, 1, B>, dbcdef_kernel<256, 4, 3, B>,
                            dbcdef_kernel<256, 4, 0, B, true>, dbcdef_kernel<256, 4, 1, B, true>,
                            dbcdef_kernel<256, 4, 3, B, true>, dbcdef_kernel<128, 5, 0, B>, dbcdef_kernel<128, 5, 1, B>,
-                           dbcdef_kernel<128, 5, 3, B>})
+                           dbcdef_kernel<128, 5, 3, B>, dbcdef_kernel<512, 2, 0, B>, dbcdef_kernel<512, 2, 1, B>,
+                           dbcdef_kernel<512, 2, 3, B>, dbcdef_kernel<512, 2, 0, B, true>,
+                           dbcdef_kernel<512, 2, 1, B, true>, dbcdef_kernel<512, 2, 3, B, true>})
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(k, attr, kMaxSmem);
             for (auto k : {dbcdef_batch_kernel<256, 3, -1, B>, dbcdef_batch_kernel<256, 3, 0, B>,
                            dbcdef_batch_kernel<256, 3, 1, B>, dbcdef_batch_kernel<256, 3, 3, B>,
@@ -824,28 +844,31 @@ cudaError_t dbcdef_kernel_attributes() {
 
 // One kernel per chroma layout (4:4:4 and monochrome, 4:2:2, 4:2:0) and block
 // form (half-precision CDEF taps up to 10 bits, integer ones above); a frame
-// with a plane written straight to the output takes the 256-thread body that
-// does so, whatever the threads per tile.
-template <class Block>
-static cudaError_t launch_dbcdef_as(const DbCdefArgs& a, bool direct, int threads, dim3 grid, size_t smem,
-                                    cudaStream_t stream) {
+// with a plane written straight to the output takes a body that does so.
+template <int NT, int MIN_CTAS, class Block, bool DIRECT>
+static cudaError_t launch_dbcdef_nt(const DbCdefArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     const int layout = a.ssx | a.ssy << 1;
-    if (direct) {
-        auto k = layout == 3   ? dbcdef_kernel<256, 4, 3, Block, true>
-                 : layout == 1 ? dbcdef_kernel<256, 4, 1, Block, true>
-                               : dbcdef_kernel<256, 4, 0, Block, true>;
-        return launch_overlapped(k, grid, dim3(256), smem, stream, a);
-    }
-    if (threads == 128) {
-        auto k = layout == 3   ? dbcdef_kernel<128, 5, 3, Block>
-                 : layout == 1 ? dbcdef_kernel<128, 5, 1, Block>
-                               : dbcdef_kernel<128, 5, 0, Block>;
-        return launch_overlapped(k, grid, dim3(128), smem, stream, a);
-    }
-    auto k = layout == 3   ? dbcdef_kernel<256, 4, 3, Block>
-             : layout == 1 ? dbcdef_kernel<256, 4, 1, Block>
-                           : dbcdef_kernel<256, 4, 0, Block>;
-    return launch_overlapped(k, grid, dim3(256), smem, stream, a);
+    auto k = layout == 3   ? dbcdef_kernel<NT, MIN_CTAS, 3, Block, DIRECT>
+             : layout == 1 ? dbcdef_kernel<NT, MIN_CTAS, 1, Block, DIRECT>
+                           : dbcdef_kernel<NT, MIN_CTAS, 0, Block, DIRECT>;
+    return launch_overlapped(k, grid, dim3(NT), smem, stream, a);
+}
+
+template <class Block>
+static cudaError_t launch_dbcdef_as(const DbCdefArgs& a, bool direct, int threads, int sm_count, dim3 grid,
+                                    size_t smem, cudaStream_t stream) {
+    // A frame whose tiles are all resident at 512 threads each (two CTAs per
+    // SM) takes one tile's latency, which the second set of warps shortens:
+    // 640x360 23.0 -> 18.2 us, 1280x720 26.1 -> 23.6 us.  With more tiles than
+    // that a CTA per SM more is the better use of the registers: 1440x810
+    // (299 tiles) 27.5 us at 256 threads, 31.5 at 512.  (1024 threads, one CTA
+    // per SM: 17.7 us at 640x360, 30.0 at 1280x720.)
+    if (threads != 128 && (long)grid.x * grid.y <= 2L * sm_count)
+        return direct ? launch_dbcdef_nt<512, 2, Block, true>(a, grid, smem, stream)
+                      : launch_dbcdef_nt<512, 2, Block, false>(a, grid, smem, stream);
+    if (direct) return launch_dbcdef_nt<256, 4, Block, true>(a, grid, smem, stream);
+    if (threads == 128) return launch_dbcdef_nt<128, 5, Block, false>(a, grid, smem, stream);
+    return launch_dbcdef_nt<256, 4, Block, false>(a, grid, smem, stream);
 }
 
 cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream) {
@@ -855,8 +878,8 @@ cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     const dim3 grid(div_up(L.info.mi_cols, 16), div_up(L.info.mi_rows, 16));
     const bool direct = a.direct[0].out.data || a.direct[1].out.data || a.direct[2].out.data;
-    return a.bit_depth <= 10 ? launch_dbcdef_as<HalfBlock>(a, direct, L.threads, grid, smem, stream)
-                             : launch_dbcdef_as<PairBlock>(a, direct, L.threads, grid, smem, stream);
+    return a.bit_depth <= 10 ? launch_dbcdef_as<HalfBlock>(a, direct, L.threads, L.sm_count, grid, smem, stream)
+                             : launch_dbcdef_as<PairBlock>(a, direct, L.threads, L.sm_count, grid, smem, stream);
 }
 
 template <class Block>

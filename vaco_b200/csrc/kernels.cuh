@@ -153,7 +153,8 @@ struct DbCdefLaunch {
     int cdef_stride, cdef_count;
     vaco_av1_cdef_params cdef;
     DeviceStatus* status;
-    int threads = 256;          // threads per tile: 256 or 128
+    int threads = 256;          // threads per tile: 256 (512 for frames of few tiles) or 128
+    int sm_count = 0;
     DirectPlane direct[3] = {};  // per plane; all off unless set
 };
 cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream);
