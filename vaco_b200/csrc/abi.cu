@@ -82,19 +82,36 @@ int32_t invalid(int32_t* msg, int m) {
                                                                                 : VACO_AV1_INVALID_DATA;
 }
 
+// Starts a call from a clean status word.  The word is clean unless its flag
+// is up (a call that failed half-way left its kernels' report unread), or the
+// context defers status: then it may hold earlier frames' errors, which a call
+// that returns its own status drops.
 cudaError_t reset_status(vaco_av1_ctx* ctx, cudaStream_t s) {
-    return cudaMemsetAsync(ctx->status, 0xFF, sizeof(DeviceStatus), s);
+    if (!ctx->deferred && *ctx->status_flag == 0) return cudaSuccess;
+    if (!ctx->deferred) {
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return e;
+        *ctx->status_flag = 0;
+    }
+    return cudaMemsetAsync(ctx->status, 0xFF, sizeof(unsigned long long), s);
 }
 
-// Read the status word back (one small D2H copy + stream sync) and fold in
-// the earliest host-detected error `host_key`.
+// Waits for the stream, reads the status word back when a kernel raised its
+// flag, and folds in the earliest host-detected error `host_key`.
 int32_t finish(vaco_av1_ctx* ctx, cudaStream_t s, unsigned long long host_key, int32_t* msg) {
-    cudaError_t e = cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+    unsigned long long key = kNoError;
+    if (*ctx->status_flag) {
+        e = cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess && !ctx->deferred)
+            e = cudaMemsetAsync(ctx->status, 0xFF, sizeof(unsigned long long), s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+        if (!ctx->deferred) *ctx->status_flag = 0;
+        key = *ctx->status_host;
+    }
     ctx->collect_marks();
-    unsigned long long key = *ctx->status_host;
     if (host_key < key) key = host_key;
     if (key == kNoError) {
         set_msg(msg, VACO_AV1_MSG_NONE);
@@ -304,6 +321,15 @@ int32_t vaco_av1_ctx_create(int32_t device, vaco_av1_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&c->status, sizeof(DeviceStatus));
     if (e == cudaSuccess) e = cudaMallocHost(&c->status_host, sizeof(unsigned long long));
+    void* flag = nullptr;
+    if (e == cudaSuccess) e = cudaMallocHost(&flag, sizeof(unsigned));
+    c->status_flag = static_cast<volatile unsigned*>(flag);
+    if (e == cudaSuccess) {
+        *c->status_flag = 0;
+        const DeviceStatus clean{kNoError, static_cast<unsigned*>(flag)};
+        e = cudaMemcpyAsync(c->status, &clean, sizeof clean, cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    }
     if (e != cudaSuccess) {
         vaco_av1_ctx_destroy(c);
         return VACO_AV1_DEVICE_ERROR;
@@ -337,12 +363,13 @@ void vaco_av1_ctx_destroy(vaco_av1_ctx* ctx) {
     if (ctx->copy_out) cudaStreamDestroy(ctx->copy_out);
     if (ctx->status) cudaFree(ctx->status);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
+    if (ctx->status_flag) cudaFreeHost(const_cast<unsigned*>(ctx->status_flag));
     for (auto& frame : ctx->marks)
         for (auto& ev : frame)
             if (ev) cudaEventDestroy(ev);
     for (auto& g : ctx->graphs) cudaGraphExecDestroy(g.second);
     if (ctx->batch_table_host) cudaFreeHost(ctx->batch_table_host);
-    if (ctx->batch_status_host) cudaFreeHost(ctx->batch_status_host);
+    if (ctx->batch_flag) cudaFreeHost(const_cast<unsigned*>(ctx->batch_flag));
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -354,8 +381,10 @@ int32_t vaco_av1_ctx_set_deferred_status(vaco_av1_ctx* ctx, int32_t enable) {
     if (!ctx) return VACO_AV1_INVALID_DATA;
     cudaSetDevice(ctx->device);
     // Start from a clean word; the caller has no work of this context in flight.
-    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemset(ctx->status, 0xFF, sizeof(DeviceStatus)) != cudaSuccess)
+    if (cudaDeviceSynchronize() != cudaSuccess ||
+        cudaMemset(ctx->status, 0xFF, sizeof(unsigned long long)) != cudaSuccess)
         return VACO_AV1_DEVICE_ERROR;
+    *ctx->status_flag = 0;
     ctx->deferred = enable != 0;
     return VACO_AV1_OK;
 }
@@ -365,10 +394,11 @@ int32_t vaco_av1_ctx_flush(vaco_av1_ctx* ctx, void* stream, int32_t* msg) {
     cudaSetDevice(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
     const int32_t st = finish(ctx, s, kNoError, msg);
-    if (st == VACO_AV1_DEVICE_ERROR) return st;
+    if (st == VACO_AV1_DEVICE_ERROR || *ctx->status_flag == 0) return st;
     cudaError_t e = reset_status(ctx, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+    *ctx->status_flag = 0;
     return st;
 }
 
@@ -1141,6 +1171,7 @@ int32_t vaco_av1_postfilter_frame_host_submit(vaco_av1_ctx* ctx, const vaco_av1_
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&slot.filtered, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaMalloc(&slot.status, sizeof(DeviceStatus));
+        if (e == cudaSuccess) e = cudaMemsetAsync(slot.status, 0, sizeof(DeviceStatus), ctx->stream);  // no host flag
         if (e == cudaSuccess) e = cudaMallocHost(&slot.status_host, sizeof(unsigned long long));
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
@@ -1149,7 +1180,7 @@ int32_t vaco_av1_postfilter_frame_host_submit(vaco_av1_ctx* ctx, const vaco_av1_
     ctx->scratch_set = 1 + k;
     ctx->status = slot.status;
     cudaStream_t s = ctx->stream;
-    e = cudaMemsetAsync(slot.status, 0xFF, sizeof(DeviceStatus), s);
+    e = cudaMemsetAsync(slot.status, 0xFF, sizeof(unsigned long long), s);
     vaco_av1_picture dst{};
     int32_t st = e == cudaSuccess ? postfilter_from_host(ctx, s, job, &dst, msg, ctx->copy_in, slot.staged, true)
                                   : cuda_fail(ctx, e, msg);

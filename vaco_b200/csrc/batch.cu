@@ -11,7 +11,7 @@
 //   4. one restoration kernel over all frames' tiles (restoration.cu), which
 //      also validates every restoration unit and copies planes whose
 //      frame-level restoration is off
-//   5. one download of the per-frame status words
+//   5. the per-frame status words, read only when a kernel raised the batch flag
 // With tuning.use_graphs, steps 1-5 are captured once per batch composition as
 // a CUDA graph and replayed afterwards; the tables carry every per-batch
 // pointer, so a replay only needs the host to refresh the pinned staging copy.
@@ -336,18 +336,18 @@ int32_t vaco::batch_enqueue(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_fr
         ctx->batch_table_host_bytes = table_bytes;
         ++ctx->scratch_generation;
     }
-    if (ctx->batch_status_host_count < (size_t)n) {
-        if (ctx->batch_status_host) cudaFreeHost(ctx->batch_status_host);
-        ctx->batch_status_host = nullptr;
-        ctx->batch_status_host_count = 0;
-        e = cudaMallocHost(&ctx->batch_status_host, sizeof(unsigned long long) * n);
+    if (!ctx->batch_flag) {
+        void* flag = nullptr;
+        e = cudaMallocHost(&flag, sizeof(unsigned));
         if (e != cudaSuccess) return fail(ctx, e, statuses, msgs, n);
-        ctx->batch_status_host_count = n;
-        ++ctx->scratch_generation;
+        ctx->batch_flag = static_cast<volatile unsigned*>(flag);
     }
+    *ctx->batch_flag = 0;  // the context's previous batch has been collected
     unsigned char* htab = ctx->batch_table_host;
     DeviceStatus* dstatus = reinterpret_cast<DeviceStatus*>(dtab + off_status);
-    memset(htab + off_status, 0xFF, sizeof(DeviceStatus) * n);
+    for (int i = 0; i < n; ++i)
+        reinterpret_cast<DeviceStatus*>(htab + off_status)[i] =
+            DeviceStatus{kNoError, const_cast<unsigned*>(ctx->batch_flag)};
 
     // deblock + CDEF records
     size_t smem_db = 0;
@@ -499,9 +499,6 @@ int32_t vaco::batch_enqueue(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_fr
             r = launch_restoration_batch(dtab + off_lr, reinterpret_cast<const int*>(dtab + off_lr_prefix),
                                          (int)lr_order.size(), lr_prefix[lr_order.size()], ctx->tuning.lr_ctas_per_sm,
                                          s);
-        if (r == cudaSuccess)
-            r = cudaMemcpyAsync(ctx->batch_status_host, dstatus, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost,
-                                s);
         return r;
     };
     // kernel launches of this batch: deblock+CDEF, superres, restoration
@@ -547,6 +544,7 @@ int32_t vaco::batch_enqueue(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_fr
     if (e == cudaSuccess) ctx->mark(1, s), ctx->mark(2, s), ctx->mark(3, s), ctx->mark(4, s);
     if (e != cudaSuccess) return fail(ctx, e, statuses, msgs, n);
     pending->n = n;
+    pending->words = dstatus;
     pending->host_keys.resize(n);
     pending->queued.resize(n);
     for (int i = 0; i < n; ++i) {
@@ -559,9 +557,17 @@ int32_t vaco::batch_enqueue(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_fr
 // Per-frame results of a batch whose stream work has completed.
 int32_t vaco::batch_collect(vaco_av1_ctx* ctx, const BatchPending& pending, int32_t* statuses, int32_t* msgs) {
     ctx->collect_marks();
+    std::vector<DeviceStatus> words;
+    if (*ctx->batch_flag) {  // some frame failed: read every frame's word
+        words.resize(pending.n);
+        cudaError_t e = cudaMemcpyAsync(words.data(), pending.words, sizeof(DeviceStatus) * pending.n,
+                                        cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return fail(ctx, e, statuses, msgs, pending.n);
+    }
     int32_t first = VACO_AV1_OK;
     for (int i = 0; i < pending.n; ++i) {
-        unsigned long long key = pending.queued[i] ? ctx->batch_status_host[i] : kNoError;
+        unsigned long long key = pending.queued[i] && !words.empty() ? words[i].first_error : kNoError;
         if (pending.host_keys[i] < key) key = pending.host_keys[i];
         const int32_t st = key == kNoError ? VACO_AV1_OK : VACO_AV1_INVALID_DATA;
         if (statuses) statuses[i] = st;

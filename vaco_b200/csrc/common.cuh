@@ -15,9 +15,14 @@ namespace vaco {
 //   bits 63..8  ordering key (stage, then the raster position vaco would have
 //               reached the failing check at), bits 7..0  vaco_av1_msg
 // Kernels atomicMin it, so the host reads the error vaco itself would have
-// returned first.  ~0 means "no error".
+// returned first.  ~0 means "no error".  The first report also raises a flag
+// in page-locked host memory, so a host that has waited for the work knows
+// without a copy that there is nothing to read: a device-to-host copy of the
+// word behind the kernels cost 5 to 10 us a call, depending on when the copy
+// engine woke up, and resetting the word another 2.
 struct DeviceStatus {
     unsigned long long first_error;
+    unsigned* host_flag;  // may be null
 };
 
 constexpr unsigned long long kNoError = ~0ull;
@@ -30,6 +35,7 @@ __device__ __forceinline__ void report_error(DeviceStatus* st, unsigned stage,
                                              unsigned long long position, unsigned msg) {
     unsigned long long key = ((unsigned long long)stage << 60) | ((position & ((1ull << 52) - 1)) << 8) | msg;
     atomicMin(&st->first_error, key);
+    if (st->host_flag) *static_cast<volatile unsigned*>(st->host_flag) = 1u;
 }
 
 // ---------------------------------------------------------------- overlapped launches

@@ -18,6 +18,9 @@ struct vaco_av1_ctx {
     cudaStream_t stream = nullptr;
     vaco::DeviceStatus* status = nullptr;     // device
     unsigned long long* status_host = nullptr;  // pinned
+    // Raised by the kernels that report into `status` (see DeviceStatus).
+    // While it is down the word holds "no error", so nothing resets it.
+    volatile unsigned* status_flag = nullptr;   // pinned
     int last_cuda_error = 0;
     uint64_t launches = 0;
     // deferred status (vaco_av1_ctx_set_deferred_status): chain calls on
@@ -103,8 +106,7 @@ struct vaco_av1_ctx {
     vaco_av1_tuning tuning = {3, 4, 1, 1, 256, 1};
     unsigned char* batch_table_host = nullptr;   // pinned staging of the per-batch tables
     size_t batch_table_host_bytes = 0;
-    unsigned long long* batch_status_host = nullptr;  // pinned copy of the per-frame status words
-    size_t batch_status_host_count = 0;
+    volatile unsigned* batch_flag = nullptr;     // pinned: some frame of the batch reported an error
     std::map<std::string, cudaGraphExec_t> graphs;   // by batch composition (and scratch generation)
     unsigned long long scratch_generation = 0;       // bumps whenever a scratch slot is reallocated
     int sm_count = 0;
@@ -152,6 +154,7 @@ struct BatchPending {
     int n = 0;
     std::vector<unsigned long long> host_keys;
     std::vector<int> queued;  // frames whose device status word is live
+    const DeviceStatus* words = nullptr;  // device, one per frame
 };
 int32_t batch_enqueue(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_frame_job* jobs, int n, BatchPending* pending);
 int32_t batch_collect(vaco_av1_ctx* ctx, const BatchPending& pending, int32_t* statuses, int32_t* msgs);

@@ -163,7 +163,8 @@ extern "C" int32_t vaco_av1_postfilter_frame_noalloc(void* stream, const vaco_av
     if (!fits) return fail(msg, VACO_AV1_LIMIT_EXCEEDED, VACO_AV1_MSG_SCRATCH_LIMIT);
 
     // Clear the status word before any kernel of this call.
-    e = cudaMemsetAsync(status, 0xFF, sizeof(DeviceStatus), s);
+    e = cudaMemsetAsync(status, 0, sizeof(DeviceStatus), s);  // no host flag
+    if (e == cudaSuccess) e = cudaMemsetAsync(status, 0xFF, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return fail(msg, VACO_AV1_DEVICE_ERROR, VACO_AV1_MSG_CUDA);
     unsigned long long host_key = kNoError;
 
