@@ -1401,11 +1401,17 @@ static int32_t film_grain_impl(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1
     }
     const int bd = info->bit_depth, ssx = info->subsampling_x, ssy = info->subsampling_y;
     if (params->apply_grain) {
-        if (gs.used) e = cudaStreamWaitEvent(gs.stream, gs.free, 0);
-        if (e == cudaSuccess) e = launch_grain_template(*params, gauss, np, bd, ssx, ssy, w, h, ws, gs.stream);
+        // Deferred frames run back to back: their templates go ahead on the
+        // sets' own streams.  A call that waits for its frame has nothing to
+        // overlap, and both kernels go to its stream.
+        cudaStream_t ts = defer ? gs.stream : s;
+        if (gs.used) e = cudaStreamWaitEvent(ts, gs.free, 0);
+        if (e == cudaSuccess) e = launch_grain_template(*params, gauss, np, bd, ssx, ssy, w, h, ws, ts);
         ctx->launches++;
-        if (e == cudaSuccess) e = cudaEventRecord(gs.ready, gs.stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, gs.ready, 0);
+        if (defer) {
+            if (e == cudaSuccess) e = cudaEventRecord(gs.ready, ts);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(s, gs.ready, 0);
+        }
     }
     if (e == cudaSuccess) e = launch_grain_apply(*params, din, dout, np, bd, ssx, ssy, w, h, ws, ctx->status,
                                                  ctx->sm_count, s);
