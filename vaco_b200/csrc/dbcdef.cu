@@ -59,9 +59,10 @@ constexpr int kShiftWords = kShiftRows * (64 + 2 * kHalo) / 2 + 2 * (32 + 2 * kH
 // levels at luma cells up to row and column 17.
 constexpr int kWinTop = 3, kWinLeft = 2, kWinRows = 22, kWinCols = 20, kWinCells = kWinRows * kWinCols;
 struct SideWindow {
-    uint8_t tx[2][kWinCells];  // luma, chroma TX_SIZE
+    uint8_t tx[2][kWinCells];  // luma, chroma transform sizes: log2 width | log2 height << 4
     uint32_t lvl[kWinCells];   // loop-filter levels (Yv, Yh, U, V) when a level map is given
 };
+__device__ __forceinline__ uint8_t tx_logs(int t) { return (uint8_t)(tx_w_log2(t) | tx_h_log2(t) << 4); }
 
 // n / d for the tile loops' small quotients (segments per edge row 9, 10,
 // 17, 18; 16-byte vectors per staged row 6, 10; sentinel window widths 36,
@@ -266,78 +267,59 @@ __device__ __forceinline__ void deblock_lists(const DbCdefArgs& a, int ssx, int 
     const PlaneGeom gl = plane_geom(0, ssx, ssy), gc = plane_geom(1, ssx, ssy);
     const int nrl = gl.th / 4 + 4, ncl = gl.tw / 4 + 2;  // luma cells: rows, columns
     const int nrc = gc.th / 4 + 2, ncc = gc.tw / 4 + 2;  // chroma
-    const int n0 = nrl * ncl, nc = a.num_planes > 1 ? nrc * ncc : 0;
+    const bool u_on = a.num_planes > 1 && a.levels[2] != 0, v_on = a.num_planes > 1 && a.levels[3] != 0;
+    const int n0 = nrl * ncl, n = n0 + (u_on || v_on ? nrc * ncc : 0);
     const unsigned m0 = small_div_magic(ncl), mc = small_div_magic(ncc);
     const int mi_r0 = y0 >> 2, mi_c0 = x0 >> 2;
-    for (int i = tid; i < n0 + 2 * nc; i += NT) {
-        int p = 0, j = i;
-        if (j >= n0) {
-            j -= n0;
-            p = 1;
-            if (j >= nc) {
-                j -= nc;
-                p = 2;
-            }
-        }
-        if (p != 0 && a.levels[1 + p] == 0) continue;
-        const PlaneGeom g = p ? gc : gl;
-        const int nr = p ? nrc : nrl, ncol = p ? ncc : ncl, top = p ? 1 : 2;
-        const int cr = small_div(j, p ? mc : m0), cc = j - cr * ncol;
-        const DevPlane& P = a.dst[p];
+    for (int i = tid; i < n; i += NT) {
+        const bool chroma = i >= n0;
+        const int j = chroma ? i - n0 : i;
+        const PlaneGeom g = chroma ? gc : gl;
+        const int nr = chroma ? nrc : nrl, ncol = chroma ? ncc : ncl, top = chroma ? 1 : 2;
+        const int cr = small_div(j, chroma ? mc : m0), cc = j - cr * ncol;
+        const DevPlane& P = a.dst[chroma ? 1 : 0];
         const int px0 = x0 >> g.sx, py0 = y0 >> g.sy;
         const int yp = py0 + 4 * (cr - top), xp = px0 - 4 + 4 * cc;
         const int col = (xp >> 2) << g.sx, row = (yp >> 2) << g.sy;
         if (!(xp >= 0 && yp >= 0 && xp < P.width && yp < P.height && col * 4 < a.coded_width &&
               row * 4 < a.coded_height))
             continue;
-        const bool vert = cc >= 1 && xp > 0;                              // pass 0 candidate
-        const bool horz = cr >= top && cr - top <= g.th / 4 && yp > 0;    // pass 1 candidate
+        const uint8_t* map = side.tx[chroma ? 1 : 0];
+        const int w = (cr - top + kWinTop) * kWinCols + cc - 1 + kWinLeft;
+        const int cur = map[w], cw = cur & 15, ch = cur >> 4;
+        // transform edges on the cell's left (pass 0) and top (pass 1)
+        const bool vert = cc >= 1 && xp > 0 && (xp & ((1 << cw) - 1)) == 0;
+        const bool horz = cr >= top && cr - top <= g.th / 4 && yp > 0 && (yp & ((1 << ch) - 1)) == 0;
         if (!vert && !horz) continue;
-        const uint8_t* map = side.tx[p ? 1 : 0];
-        const int w = (((yp - py0) >> 2) + kWinTop) * kWinCols + ((xp - px0) >> 2) + kWinLeft;  // multiples of 4
-        const int cur = map[w];
         const int r = row | g.sy, c = col | g.sx;
         const int lw = (r - mi_r0 + kWinTop) * kWinCols + c - mi_c0 + kWinLeft;
         const uint32_t lv = a.lvl_map ? side.lvl[lw] : 0;
         const int off = (yp - py0 + kHalo) * g.pitch + (xp - px0 + kHalo);
-        if (vert) {
-            const int cl = tx_w_log2(cur), pl = tx_w_log2(map[w - 1]);
-            if ((xp & ((1 << cl) - 1)) == 0) {
-                const int li = p == 0 ? 0 : p + 1;  // level index (7.14.5)
+        // Appends the edge of filter size 1 << lg to its class list, for luma
+        // or for both chroma planes: level index li (7.14.5), from the cell
+        // before where the cell's own level is 0.
+        auto add = [&](int pass, int lg, int li, int before, bool first, bool last) {
+            const int cls = lg == 2 ? 0 : chroma ? 1 : lg == 3 ? 2 : 3;
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                if (v && !chroma) break;
+                if (chroma && !(v ? v_on : u_on)) continue;
                 int lvl;
                 if (a.lvl_map) {
-                    lvl = (lv >> (8 * li)) & 0xFF;
-                    if (lvl == 0) lvl = (side.lvl[lw - (1 << g.sx)] >> (8 * li)) & 0xFF;
+                    lvl = (lv >> (8 * (li + v))) & 0xFF;
+                    if (lvl == 0) lvl = (side.lvl[before] >> (8 * (li + v))) & 0xFF;
                 } else {
-                    lvl = a.levels[li];
+                    lvl = a.levels[li + v];
                 }
-                if (lvl != 0) {
-                    const int size = min(p ? 8 : 16, 1 << min(cl, pl));
-                    const int cls = size == 4 ? 0 : p ? 1 : size == 8 ? 2 : 3;
-                    const int at = atomicAdd(&s_count[cls], 1);
-                    s_list[c_list_off[cls] + at] = seg_entry(lvl, off, p, cr == 0, cr == nr - 1);
-                }
+                if (lvl == 0) continue;
+                const int at = atomicAdd(&s_count[4 * pass + cls], 1);
+                s_list[pass * kListTotal + c_list_off[cls] + at] =
+                    seg_entry(lvl, off, chroma ? 1 + v : 0, first, last);
             }
-        }
-        if (horz) {
-            const int cl = tx_h_log2(cur), pl = tx_h_log2(map[w - kWinCols]);
-            if ((yp & ((1 << cl) - 1)) == 0) {
-                const int li = p == 0 ? 1 : p + 1;
-                int lvl;
-                if (a.lvl_map) {
-                    lvl = (lv >> (8 * li)) & 0xFF;
-                    if (lvl == 0) lvl = (side.lvl[lw - (kWinCols << g.sy)] >> (8 * li)) & 0xFF;
-                } else {
-                    lvl = a.levels[li];
-                }
-                if (lvl != 0) {
-                    const int size = min(p ? 8 : 16, 1 << min(cl, pl));
-                    const int cls = size == 4 ? 0 : p ? 1 : size == 8 ? 2 : 3;
-                    const int at = atomicAdd(&s_count[4 + cls], 1);
-                    s_list[kListTotal + c_list_off[cls] + at] = seg_entry(lvl, off, p, cc == 0, cc == ncol - 1);
-                }
-            }
-        }
+        };
+        if (vert) add(0, min(cw, map[w - 1] & 15), chroma ? 2 : 0, lw - (1 << g.sx), cr == 0, cr == nr - 1);
+        if (horz) add(1, min(ch, map[w - kWinCols] >> 4), chroma ? 2 : 1, lw - (kWinCols << g.sy), cc == 0,
+                      cc == ncol - 1);
     }
 }
 
@@ -453,12 +435,34 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     // sample.  Rows past the top/bottom edge repeat the edge row.  (Staging
     // interior tiles with 2-D tensor copies instead measured 1.4 % slower
     // for the whole chain: the extra path costs more than the copies save.)
+    // A tile whose halo lies inside every plane (nine in ten of a 4K frame)
+    // steps down its columns by pointer increments alone.
+    auto inside = [&](int p) {
+        const PlaneGeom g = plane_geom(p, ssx, ssy);
+        const int px0 = x0 >> g.sx, py0 = y0 >> g.sy;
+        return px0 >= kHalo && py0 >= kHalo && px0 + g.tw + kHalo <= a.src[p].width &&
+               py0 + g.th + kHalo <= a.src[p].height;
+    };
+    const bool interior = a.vec_ok && inside(0) && (a.num_planes == 1 || inside(1));
     for (int p = 0; p < a.num_planes; ++p) {
         const PlaneGeom g = plane_geom(p, ssx, ssy);
         const DevPlaneC& P = a.src[p];
         uint16_t* t = smem + a.plane_off[p];
         const int px0 = x0 >> g.sx, py0 = y0 >> g.sy;
         const int vpr = g.pitch / 8;
+        if (interior) {
+            const int step = NT / vpr, r0 = tid / vpr, cv = tid - r0 * vpr;  // vpr is 10 or 6
+            if (r0 >= step) continue;
+            const uint16_t* src = P.data + (long)(py0 - kHalo + r0) * P.stride + px0 - kHalo + cv * 8;
+            unsigned dst = (unsigned)__cvta_generic_to_shared(t + r0 * g.pitch + cv * 8);
+            const long src_step = (long)step * P.stride;
+            for (int r = r0; r < g.rows; r += step) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+                src += src_step;
+                dst += (unsigned)(step * g.pitch * 2);
+            }
+            continue;
+        }
         const unsigned mv = small_div_magic(vpr);
         for (int v = tid; v < g.rows * vpr; v += NT) {
             const int r = small_div(v, mv), cv = v - r * vpr;
@@ -478,52 +482,40 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 
     // ---- the side information the deblocking decisions read, while the
-    // copies are in flight (cells the two passes touch; see SideWindow)
+    // copies are in flight (cells the two passes touch; see SideWindow).  Each
+    // cell is checked where it is loaded: the windows of all tiles together
+    // hold exactly the maps' cells.
     {
         const int crows = (a.mi_rows + ssy) >> ssy, ccols = (a.mi_cols + ssx) >> ssx;
         const int cr0 = (mi_r0 >> ssy) - kWinTop, cc0 = (mi_c0 >> ssx) - kWinLeft;
+        int bad = 0;
         for (int i = tid; i < kWinCells; i += NT) {
             const int wr = i / kWinCols, wc = i - wr * kWinCols;
             const int r = mi_r0 - kWinTop + wr, c = mi_c0 - kWinLeft + wc;
             if (r >= 0 && c >= 0 && r < a.mi_rows && c < a.mi_cols) {
                 const long cell = (long)r * a.mi_cols + c;
-                s_side.tx[0][i] = __ldg(a.tx_luma + cell);
-                if (a.lvl_map) s_side.lvl[i] = __ldg(reinterpret_cast<const uint32_t*>(a.lvl_map) + cell);
-            }
-            if (a.num_planes > 1 && cr0 + wr >= 0 && cc0 + wc >= 0 && cr0 + wr < crows && cc0 + wc < ccols)
-                s_side.tx[1][i] = __ldg(a.tx_chroma + (long)(cr0 + wr) * ccols + cc0 + wc);
-        }
-    }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    const bool any_active = __syncthreads_or(act);
-
-    // ---- input checks from shared memory: the tile's own cells (transform
-    // sizes, levels) and the tile's own samples
-    {
-        int bad = 0;
-        for (int i = tid; i < 256; i += NT) {
-            const int r = mi_r0 + (i >> 4), c = mi_c0 + (i & 15);
-            if (r < a.mi_rows && c < a.mi_cols) {
-                const int w = (i >> 4) + kWinTop, wc = (i & 15) + kWinLeft;
-                bad |= s_side.tx[0][w * kWinCols + wc] > 18;
+                const int t = __ldg(a.tx_luma + cell);
+                s_side.tx[0][i] = tx_logs(t);
+                bad |= t > 18;
                 if (a.lvl_map) {
-                    const uint32_t v = s_side.lvl[w * kWinCols + wc];
-                    bad |= ((v & 0xFF) > 63) | (((v >> 8) & 0xFF) > 63) | (((v >> 16) & 0xFF) > 63) | ((v >> 24) > 63);
+                    const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(a.lvl_map) + cell);
+                    s_side.lvl[i] = v;
+                    bad |= (v & 0xC0C0C0C0u) != 0;  // a level above 63
                 }
             }
-        }
-        if (a.num_planes > 1) {
-            const int ccols = (a.mi_cols + ssx) >> ssx, crows = (a.mi_rows + ssy) >> ssy;
-            const int cw = 16 >> ssx, ch = 16 >> ssy;
-            for (int i = tid; i < cw * ch; i += NT) {
-                const int dr = i >> (4 - ssx), dc = i - dr * cw;  // cw = 16 >> ssx
-                const int r = (mi_r0 >> ssy) + dr, c = (mi_c0 >> ssx) + dc;
-                if (r < crows && c < ccols) bad |= s_side.tx[1][(dr + kWinTop) * kWinCols + dc + kWinLeft] > 18;
+            if (a.num_planes > 1 && cr0 + wr >= 0 && cc0 + wc >= 0 && cr0 + wr < crows && cc0 + wc < ccols) {
+                const int t = __ldg(a.tx_chroma + (long)(cr0 + wr) * ccols + cc0 + wc);
+                s_side.tx[1][i] = tx_logs(t);
+                bad |= t > 18;
             }
         }
         if (bad) report_error(a.status, STAGE_DEBLOCK, 0, VACO_AV1_MSG_DB_PARAMS);
     }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    const bool any_active = __syncthreads_or(act);
+
     {
+        // ---- input check from shared memory
         // Every staged sample, halo included: the halo holds samples of the
         // same planes (edge-clamped copies past their borders), so the tiles
         // together check exactly the planes' samples, and a flat pass over
@@ -550,28 +542,27 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         __syncthreads();
     }
 
-    // ---- stripe-boundary rows of the deblocked picture for restoration:
-    // rows y with (y + offset + 2) mod stripe < 4, stored at 4*boundary + that
-    // remainder (boundary = (y + offset + 2) / stripe >= 1).
-    for (int p = 0; p < a.num_planes; ++p) {
-        const DevPlane& R = a.pre_rows[p];
-        if (!R.data) continue;
-        const PlaneGeom g = plane_geom(p, ssx, ssy);
-        const int sh = 64 >> g.sy, off = 8 >> g.sy;
-        const int px0 = x0 >> g.sx, py0 = y0 >> g.sy;
-        const uint16_t* src = smem + a.plane_off[p];
-        const int width = a.dst[p].width, height = a.dst[p].height;
-        // the tile (th rows, th a multiple of the stripe height or half of it)
-        // holds boundary rows y = k*sh - off - 2 + sub, sub < 4
-        const int lsh = 6 - g.sy;  // log2 of the stripe height
-        for (int i = warp; i < 4 * ((g.th >> lsh) + 1); i += kWarpsNT) {
-            const int kk = i >> 2, sub = i & 3;
-            const int kb = ((py0 + off + 2) >> lsh) + kk;
-            const int y = kb * sh - off - 2 + sub;
-            if (kb < 1 || y < py0 || y >= py0 + g.th || y >= height) continue;
-            for (int c = lane; c < g.tw; c += 32)
-                if (px0 + c < width)
-                    R.data[(long)(4 * kb + sub) * R.stride + px0 + c] = src[(y - py0 + kHalo) * g.pitch + c + kHalo];
+    // ---- stripe-boundary rows of the deblocked picture for restoration: rows
+    // y with (y + offset + 2) mod stripe < 4, stored at 4*boundary + that
+    // remainder (boundary = (y + offset + 2) / stripe >= 1).  A tile is one
+    // stripe high, so it holds the four rows around its own boundary, from row
+    // th - offset - 2 on: 8-sample vectors, one a thread (64 for 4:2:0).  The
+    // compact buffers' rows are padded to 64 samples, which takes the vector
+    // that a 4:2:0 chroma plane's last columns share with the padding.
+    {
+        constexpr int nl = 64 / 8, kMost = 3 * nl;  // vectors of a row: luma's, all planes' at most
+        const int ncv = a.num_planes > 1 ? (64 >> ssx) / 8 : 0;
+        const int sub_row = tid / kMost, i = tid - sub_row * kMost;
+        if (tid < 4 * kMost && i < nl + 2 * ncv) {
+            const int p = i < nl ? 0 : i < nl + ncv ? 1 : 2;
+            const int c = 8 * (i - (p == 0 ? 0 : nl + (p - 1) * ncv));
+            const DevPlane& R = a.pre_rows[p];
+            const PlaneGeom g = plane_geom(p ? 1 : 0, ssx, ssy);
+            const int off = 8 >> g.sy, px0 = x0 >> g.sx, py0 = y0 >> g.sy;
+            const int r = g.th - off - 2 + sub_row;
+            if (R.data && px0 + c < a.dst[p].width && py0 + r < a.dst[p].height)
+                *reinterpret_cast<uint4*>(R.data + (long)(4 * (py0 / g.th + 1) + sub_row) * R.stride + px0 + c) =
+                    *reinterpret_cast<const uint4*>(smem + a.plane_off[p] + (r + kHalo) * g.pitch + kHalo + c);
         }
     }
 
