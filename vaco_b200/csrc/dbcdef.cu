@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 
 #include "cdef_core.cuh"
 #include "common.cuh"
@@ -338,7 +339,7 @@ __device__ __forceinline__ void deblock_lists(const DbCdefArgs& a, int ssx, int 
 // and, for chroma and size 4, 3.  So there are no clamped reads.  (A second,
 // clamping body per class made the kernel 110 KB of code instead of 79 KB and
 // a 4K 10-bit frame 1.2 % slower, without ever running.)
-template <int PASS, int NT>
+template <int PASS, int NT, bool HALF>
 __device__ __forceinline__ void deblock_filter(const DbCdefArgs& a, int ssx, int ssy, uint16_t* smem,
                                                const uint32_t* s_list, const int* s_count,
                                                const PairStrength* s_str) {
@@ -373,7 +374,7 @@ __device__ __forceinline__ void deblock_filter(const DbCdefArgs& a, int ssx, int
         const int lvl = e & 63, off = (e >> 6) & 0x1FFF, p = (e >> 19) & 3;
         const int pitch = p ? gc.pitch : gl.pitch;
         uint16_t* q = smem + a.plane_off[p] + off + (PASS == 0 ? 2 * h * pitch : 2 * h);
-        filter_pair_class<PASS>(cls, q, pitch, s_str[lvl], a.bit_depth - 8);
+        filter_pair_class<PASS, HALF>(cls, q, pitch, s_str[lvl], a.bit_depth - 8);
     }
     __syncthreads();
 }
@@ -384,6 +385,7 @@ __device__ __forceinline__ void deblock_filter(const DbCdefArgs& a, int ssx, int
 template <int NT, int LAYOUT, class Block, bool DIRECT = false>
 __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int tile_y) {
     constexpr int kWarpsNT = NT / 32;
+    constexpr bool kHalf = std::is_same<Block, HalfBlock>::value;  // samples of up to 10 bits
     // chroma subsampling: LAYOUT = ssx | ssy << 1 fixes it at compile time
     // (every plane geometry below becomes a constant); LAYOUT < 0 reads it
     const int ssx = LAYOUT < 0 ? a.ssx : (LAYOUT & 1), ssy = LAYOUT < 0 ? a.ssy : (LAYOUT >> 1);
@@ -427,7 +429,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     // the deblocking lists' lengths and strengths, published by the staging
     // barrier below
     if (tid < 8) s_count[tid] = 0;
-    if (a.deblock_on && tid < 64) s_str[tid] = pair_strength(strength_of(tid, a.sharpness), a.bit_depth - 8);
+    if (a.deblock_on && tid < 64) s_str[tid] = pair_strength<kHalf>(strength_of(tid, a.sharpness), a.bit_depth - 8);
 
     // ---- every plane's tile with an 8-sample halo (edge-clamped).  Whole
     // 16-byte chunks inside the plane go by cp.async, all in flight at once;
@@ -534,8 +536,8 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     if (a.deblock_on) {
         deblock_lists<NT>(a, ssx, ssy, x0, y0, s_side, s_list, s_count);
         __syncthreads();
-        deblock_filter<0, NT>(a, ssx, ssy, smem, s_list, s_count, s_str);
-        deblock_filter<1, NT>(a, ssx, ssy, smem, s_list + kListTotal, s_count + 4, s_str);
+        deblock_filter<0, NT, kHalf>(a, ssx, ssy, smem, s_list, s_count, s_str);
+        deblock_filter<1, NT, kHalf>(a, ssx, ssy, smem, s_list + kListTotal, s_count + 4, s_str);
     } else {
         // the sample check above reads every staged sample, the sentinel
         // phase below overwrites some

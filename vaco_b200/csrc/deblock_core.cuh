@@ -172,24 +172,128 @@ __device__ __forceinline__ uint32_t sel2(uint32_t m, uint32_t a, uint32_t b) { r
 
 constexpr int kNarrowBias = 1 << 14;
 
+// ---- half-precision forms, samples of up to 10 bits
+//
+// As in the CDEF taps (cdef_core.cuh), a word of two integers up to 2048 is a
+// pair of halves in units of 2^-24 as it is.  Differences of samples are exact;
+// sums that may pass 2048 are only clamped or compared against smaller bounds
+// afterwards, which rounding, being monotonic, does not change.  Absolute
+// values are operand modifiers, and a comparison gives a lane mask in one
+// instruction, so a mask takes about a third of the integer form's
+// instructions, half of them on the FMA pipe.
+__device__ __forceinline__ uint32_t fadd2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t fsub2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t fmul2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t ffma2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t ffma2_relu(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t fabs2(uint32_t a) {
+    uint32_t d;
+    asm("abs.f16x2 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+__device__ __forceinline__ uint32_t fmin2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("min.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t fmax2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+// Per half: 0xFFFF where a > b, else 0.
+__device__ __forceinline__ uint32_t fgt2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("set.gt.u32.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// A running maximum of absolute differences, and its comparison.
+template <bool HALF>
+__device__ __forceinline__ uint32_t diff_max(uint32_t m, uint32_t a, uint32_t b) {
+    return HALF ? fmax2(m, fabs2(fsub2(a, b))) : pmax2(m, absd2(a, b));
+}
+// max(|a - b|, |c - d|)
+template <bool HALF>
+__device__ __forceinline__ uint32_t diff_max(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return HALF ? fmax2(fabs2(fsub2(a, b)), fabs2(fsub2(c, d))) : pmax2(absd2(a, b), absd2(c, d));
+}
+template <bool HALF>
+__device__ __forceinline__ uint32_t above(uint32_t a, uint32_t t) {
+    return HALF ? fgt2(a, t) : mask2(over2(a, t));
+}
+
 // Packed limit / blimit / thresh / flatness bound of a segment (7.14.4),
 // scaled to the bit depth (sh = bit depth - 8).
 struct __align__(16) PairStrength {
     uint32_t limit, blimit, thresh, one;
 };
 
+// The half form compares twice the blimit side: 2 a + (b >> 1) > L is
+// 4 a + b > 2 L + 1 for integers (b >> 1 exceeds L - 2 a exactly when b is at
+// least 2 (L - 2 a) + 2).
+template <bool HALF>
 __device__ __forceinline__ PairStrength pair_strength(const Strength& s, int sh) {
-    return PairStrength{pk2(s.limit << sh), pk2(s.blimit << sh), pk2(s.thresh << sh), pk2(1 << sh)};
+    const int blimit = s.blimit << sh;
+    return PairStrength{pk2(s.limit << sh), pk2(HALF ? 2 * blimit + 1 : blimit), pk2(s.thresh << sh), pk2(1 << sh)};
 }
 
-// 2 |p0 - q0| + |p1 - q1| / 2, the blimit side of filterMask.
-__device__ __forceinline__ uint32_t blimit_term2(const uint32_t* P, const uint32_t* Q) {
-    return absd2(P[0], Q[0]) * 2u + ((absd2(P[1], Q[1]) >> 1) & 0x7FFF7FFFu);
+// Where 2 |p0 - q0| + |p1 - q1| / 2 exceeds blimit, the blimit side of filterMask.
+template <bool HALF>
+__device__ __forceinline__ uint32_t above_blimit(const uint32_t* P, const uint32_t* Q, uint32_t blimit) {
+    if (HALF)
+        return fgt2(ffma2(fabs2(fsub2(P[0], Q[0])), 0x44004400u, fabs2(fsub2(P[1], Q[1]))), blimit);  // 4.0
+    return mask2(over2(absd2(P[0], Q[0]) * 2u + ((absd2(P[1], Q[1]) >> 1) & 0x7FFF7FFFu), blimit));
+}
+
+// The half form of narrow2().  Shifts are products that round to whole units:
+// (f + 4) >> 3 = round((2 f + 1) / 16), (f + 3) >> 3 = round((2 f - 1) / 16) and
+// (f1 + 1) >> 1 = round((2 f1 + 1) / 4), whose numerators are odd, so nothing
+// lies halfway.  Of the clamps before the shifts only the upper one can bind,
+// and it does where the shifted value would be its bound's plus one.
+__device__ __forceinline__ void narrow_half2(uint32_t& p1, uint32_t& p0, uint32_t& q0, uint32_t& q1, uint32_t hevm,
+                                             int sh) {
+    const uint32_t lo = pk2(0x8000 | 128 << sh), hi = pk2((128 << sh) - 1), top = pk2((256 << sh) - 1);
+    const uint32_t f_top = pk2(((128 << sh) - 1) >> 3);
+    uint32_t f = fmin2(fmax2(fsub2(p1, q1), lo), hi) & hevm;
+    f = fmin2(fmax2(ffma2(fsub2(q0, p0), 0x42004200u, f), lo), hi);                                // 3.0
+    const uint32_t f1 = fmin2(fmul2(ffma2(f, 0x40004000u, 0x00010001u), 0x2C002C00u), f_top);      // 2.0, 1/16
+    const uint32_t f2 = fmin2(fmul2(ffma2(f, 0x40004000u, 0x80018001u), 0x2C002C00u), f_top);
+    const uint32_t f3 = fmul2(ffma2(f1, 0x40004000u, 0x00010001u), 0x34003400u);                   // 1/4
+    q0 = fmin2(ffma2_relu(f1, 0xBC00BC00u, q0), top);                                              // -1.0
+    p0 = fmin2(ffma2_relu(f2, 0x3C003C00u, p0), top);
+    q1 = sel2(hevm, q1, fmin2(ffma2_relu(f3, 0xBC00BC00u, q1), top));
+    p1 = sel2(hevm, p1, fmin2(ffma2_relu(f3, 0x3C003C00u, p1), top));
 }
 
 // 7.14.6.3 narrow filter of both halves (hevm: 0xFFFF where hev), in place.
+template <bool HALF>
 __device__ __forceinline__ void narrow2(uint32_t& p1, uint32_t& p0, uint32_t& q0, uint32_t& q1, uint32_t hevm,
                                         int sh) {
+    if (HALF) {
+        narrow_half2(p1, p0, q0, q1, hevm, sh);
+        return;
+    }
     const int half = 0x80 << sh;
     const uint32_t lo = pk2(kNarrowBias - half), hi = pk2(kNarrowBias + half - 1);
     // f = hev ? clamp(ps1 - qs1) : 0, then clamp(f + 3 (qs0 - ps0)); biased
@@ -282,15 +386,15 @@ __device__ __forceinline__ void wide8_2(const uint32_t* P, const uint32_t* Q, ui
 }
 
 // Filter size 4: mask over p1..q1, narrow filter.
-template <int PASS>
+template <int PASS, bool HALF>
 __device__ __forceinline__ void pair_size4(uint16_t* q, int pitch, const PairStrength& s, int sh) {
     uint32_t P[2], Q[2];
     load_pair<PASS, 2>(q, pitch, P, Q);
-    const uint32_t dpq = pmax2(absd2(P[1], P[0]), absd2(Q[1], Q[0]));
-    const uint32_t keep = mask2(over2(dpq, s.limit) | over2(blimit_term2(P, Q), s.blimit));
+    const uint32_t dpq = diff_max<HALF>(P[1], P[0], Q[1], Q[0]);
+    const uint32_t keep = above<HALF>(dpq, s.limit) | above_blimit<HALF>(P, Q, s.blimit);
     if (keep == 0xFFFFFFFFu) return;
     uint32_t p1 = P[1], p0 = P[0], q0 = Q[0], q1 = Q[1];
-    narrow2(p1, p0, q0, q1, mask2(over2(dpq, s.thresh)), sh);
+    narrow2<HALF>(p1, p0, q0, q1, above<HALF>(dpq, s.thresh), sh);
     P[1] = sel2(keep, P[1], p1);
     P[0] = sel2(keep, P[0], p0);
     Q[0] = sel2(keep, Q[0], q0);
@@ -299,17 +403,17 @@ __device__ __forceinline__ void pair_size4(uint16_t* q, int pitch, const PairStr
 }
 
 // Filter size 8 on a chroma plane (filter length 6).
-template <int PASS>
+template <int PASS, bool HALF>
 __device__ __forceinline__ void pair_size6(uint16_t* q, int pitch, const PairStrength& s, int sh) {
     uint32_t P[3], Q[3];
     load_pair<PASS, 3>(q, pitch, P, Q);
-    const uint32_t dpq = pmax2(absd2(P[1], P[0]), absd2(Q[1], Q[0]));
-    const uint32_t m = pmax2(dpq, pmax2(absd2(P[2], P[1]), absd2(Q[2], Q[1])));
-    const uint32_t keep = mask2(over2(m, s.limit) | over2(blimit_term2(P, Q), s.blimit));
+    const uint32_t dpq = diff_max<HALF>(P[1], P[0], Q[1], Q[0]);
+    const uint32_t m = diff_max<HALF>(diff_max<HALF>(dpq, P[2], P[1]), Q[2], Q[1]);
+    const uint32_t keep = above<HALF>(m, s.limit) | above_blimit<HALF>(P, Q, s.blimit);
     if (keep == 0xFFFFFFFFu) return;
-    const uint32_t steep = mask2(over2(pmax2(dpq, pmax2(absd2(P[2], P[0]), absd2(Q[2], Q[0]))), s.one));
+    const uint32_t steep = above<HALF>(diff_max<HALF>(diff_max<HALF>(dpq, P[2], P[0]), Q[2], Q[0]), s.one);
     uint32_t p1 = P[1], p0 = P[0], q0 = Q[0], q1 = Q[1];
-    narrow2(p1, p0, q0, q1, mask2(over2(dpq, s.thresh)), sh);
+    narrow2<HALF>(p1, p0, q0, q1, above<HALF>(dpq, s.thresh), sh);
     if ((~steep & ~keep) != 0) {  // a flat line: the 6-tap filter
         const uint32_t p2 = P[2], q2 = Q[2], r = pk2(4), mk = 0x1FFF1FFFu;
         p1 = sel2(steep, p1, ((3u * p2 + 2u * P[1] + 2u * P[0] + Q[0] + r) >> 3) & mk);
@@ -327,27 +431,28 @@ __device__ __forceinline__ void pair_size6(uint16_t* q, int pitch, const PairStr
 }
 
 // filterMask and the flat mask over p3..q3 (filter sizes 8 and 16 on luma).
+template <bool HALF>
 __device__ __forceinline__ void masks8_2(const uint32_t* P, const uint32_t* Q, const PairStrength& s, uint32_t& dpq,
                                          uint32_t& keep, uint32_t& steep) {
-    dpq = pmax2(absd2(P[1], P[0]), absd2(Q[1], Q[0]));
-    const uint32_t m = pmax2(pmax2(dpq, pmax2(absd2(P[2], P[1]), absd2(Q[2], Q[1]))),
-                             pmax2(absd2(P[3], P[2]), absd2(Q[3], Q[2])));
-    keep = mask2(over2(m, s.limit) | over2(blimit_term2(P, Q), s.blimit));
-    const uint32_t fl = pmax2(pmax2(dpq, pmax2(absd2(P[2], P[0]), absd2(Q[2], Q[0]))),
-                              pmax2(absd2(P[3], P[0]), absd2(Q[3], Q[0])));
-    steep = mask2(over2(fl, s.one));
+    dpq = diff_max<HALF>(P[1], P[0], Q[1], Q[0]);
+    uint32_t m = diff_max<HALF>(diff_max<HALF>(dpq, P[2], P[1]), Q[2], Q[1]);
+    m = diff_max<HALF>(diff_max<HALF>(m, P[3], P[2]), Q[3], Q[2]);
+    keep = above<HALF>(m, s.limit) | above_blimit<HALF>(P, Q, s.blimit);
+    uint32_t fl = diff_max<HALF>(diff_max<HALF>(dpq, P[2], P[0]), Q[2], Q[0]);
+    fl = diff_max<HALF>(diff_max<HALF>(fl, P[3], P[0]), Q[3], Q[0]);
+    steep = above<HALF>(fl, s.one);
 }
 
 // Filter size 8 on luma (filter length 8).
-template <int PASS>
+template <int PASS, bool HALF>
 __device__ __forceinline__ void pair_size8(uint16_t* q, int pitch, const PairStrength& s, int sh) {
     uint32_t P[4], Q[4];
     load_pair<PASS, 4>(q, pitch, P, Q);
     uint32_t dpq, keep, steep;
-    masks8_2(P, Q, s, dpq, keep, steep);
+    masks8_2<HALF>(P, Q, s, dpq, keep, steep);
     if (keep == 0xFFFFFFFFu) return;
     uint32_t p1 = P[1], p0 = P[0], q0 = Q[0], q1 = Q[1];
-    narrow2(p1, p0, q0, q1, mask2(over2(dpq, s.thresh)), sh);
+    narrow2<HALF>(p1, p0, q0, q1, above<HALF>(dpq, s.thresh), sh);
     const uint32_t n[4] = {p1, p0, q0, q1};
     if ((~steep & ~keep) == 0) {  // narrow lines only: samples -2 .. 1
 #pragma unroll
@@ -375,15 +480,15 @@ __device__ __forceinline__ void pair_size8(uint16_t* q, int pitch, const PairStr
 }
 
 // Filter size 16 on luma: narrow, 8-tap or 14-tap by the flat masks.
-template <int PASS>
+template <int PASS, bool HALF>
 __device__ __forceinline__ void pair_size16(uint16_t* q, int pitch, const PairStrength& s, int sh) {
     uint32_t P[7], Q[7];
     load_pair<PASS, 7>(q, pitch, P, Q);
     uint32_t dpq, keep, steep;
-    masks8_2(P, Q, s, dpq, keep, steep);
+    masks8_2<HALF>(P, Q, s, dpq, keep, steep);
     if (keep == 0xFFFFFFFFu) return;
     uint32_t p1 = P[1], p0 = P[0], q0 = Q[0], q1 = Q[1];
-    narrow2(p1, p0, q0, q1, mask2(over2(dpq, s.thresh)), sh);
+    narrow2<HALF>(p1, p0, q0, q1, above<HALF>(dpq, s.thresh), sh);
     const uint32_t n[4] = {p1, p0, q0, q1};
     const uint32_t flat = ~steep & ~keep, narrow = steep & ~keep;
     if (flat == 0) {  // narrow lines only: samples -2 .. 1
@@ -395,10 +500,10 @@ __device__ __forceinline__ void pair_size16(uint16_t* q, int pitch, const PairSt
         store_pair<PASS, 2, 2>(q, pitch, P, Q);
         return;
     }
-    const uint32_t fl2 = pmax2(pmax2(pmax2(absd2(P[6], P[0]), absd2(Q[6], Q[0])),
-                                     pmax2(absd2(P[5], P[0]), absd2(Q[5], Q[0]))),
-                               pmax2(absd2(P[4], P[0]), absd2(Q[4], Q[0])));
-    const uint32_t flat2 = flat & ~mask2(over2(fl2, s.one)), flat1 = flat & ~flat2;
+    uint32_t fl2 = diff_max<HALF>(P[4], P[0], Q[4], Q[0]);
+#pragma unroll
+    for (int k = 5; k < 7; ++k) fl2 = diff_max<HALF>(diff_max<HALF>(fl2, P[k], P[0]), Q[k], Q[0]);
+    const uint32_t flat2 = flat & ~above<HALF>(fl2, s.one), flat1 = flat & ~flat2;
     uint32_t w[6];
     wide8_2(P, Q, w);
     uint32_t o[12];  // outputs of samples -6 .. 5
@@ -445,12 +550,12 @@ __device__ __forceinline__ void pair_size16(uint16_t* q, int pitch, const PairSt
     store_pair<PASS, PASS == 0 ? 4 : 3, PASS == 0 ? 4 : 3>(q, pitch, P, Q);
 }
 
-template <int PASS>
+template <int PASS, bool HALF>
 __device__ __forceinline__ void filter_pair_class(int cls, uint16_t* q, int pitch, const PairStrength& s, int sh) {
-    if (cls == 0) pair_size4<PASS>(q, pitch, s, sh);
-    else if (cls == 1) pair_size6<PASS>(q, pitch, s, sh);
-    else if (cls == 2) pair_size8<PASS>(q, pitch, s, sh);
-    else pair_size16<PASS>(q, pitch, s, sh);
+    if (cls == 0) pair_size4<PASS, HALF>(q, pitch, s, sh);
+    else if (cls == 1) pair_size6<PASS, HALF>(q, pitch, s, sh);
+    else if (cls == 2) pair_size8<PASS, HALF>(q, pitch, s, sh);
+    else pair_size16<PASS, HALF>(q, pitch, s, sh);
 }
 
 }  // namespace dbk
