@@ -755,7 +755,7 @@ int32_t vaco_av1_restore_plane_dev(vaco_av1_ctx* ctx, void* stream, const uint16
     p.copy_only = 0;
     p.plane_index = 0;
     p.unit_status = nullptr;  // validated by the checks above
-    e = launch_restoration(&p, 1, config->bit_depth, s);
+    e = launch_restoration(&p, 1, config->bit_depth, ctx->sm_count, s);
     ctx->launches++;
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
     e = cudaStreamSynchronize(s);
@@ -1058,7 +1058,7 @@ static int32_t postfilter_dev_impl(vaco_av1_ctx* ctx, cudaStream_t s, const vaco
         // deblocking / CDEF / superres kernels from range-checked input, so
         // they are in range by construction: no second scan is needed.
         if (hk == kNoError && nlr > 0) {
-            e = launch_restoration(lp, nlr, info.bit_depth, s);
+            e = launch_restoration(lp, nlr, info.bit_depth, ctx->sm_count, s);
             ctx->launches++;
             if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
         }

@@ -83,7 +83,7 @@ struct LrPlane {
 // A plane whose restoration is off: its tiles only copy `after` into `out`.
 LrPlane copy_only_plane(const DevPlaneC& after, const DevPlane& out, int w, int h, int sub_y, int plane_index);
 // Restores up to 3 planes in one launch.  Units must have been validated.
-cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, cudaStream_t stream);
+cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, int sm_count, cudaStream_t stream);
 // Batched form (see launch_dbcdef_batch): per-frame records of lr_args_size()
 // bytes built by build_lr_args (which returns the frame's tile count).
 size_t lr_args_size();

@@ -319,7 +319,7 @@ extern "C" int32_t vaco_av1_postfilter_frame_noalloc(void* stream, const vaco_av
             p.copy_only = 0;
         }
         if (host_key == kNoError && nlr > 0) {
-            e = launch_restoration(lp, nlr, info.bit_depth, s);
+            e = launch_restoration(lp, nlr, info.bit_depth, 0, s);
             if (e != cudaSuccess) return fail(msg, VACO_AV1_DEVICE_ERROR, VACO_AV1_MSG_CUDA);
         }
     }

@@ -34,8 +34,8 @@ namespace vaco {
 
 namespace {
 
-constexpr int kLrThreads = 256;
-constexpr int kWarps = kLrThreads / 32;
+// Threads per tile: 256, or 512 for few tiles (see launch_restoration()).
+constexpr int kLrThreads = 256, kLrThreadsFew = 512;
 constexpr int kMaxTile = 64;
 constexpr int kSPitch = kMaxTile + 16;  // staged columns x0-8 .. x0+72
 constexpr int kSRows = kMaxTile + 6;    // staged rows y0-3 .. y0+67
@@ -110,8 +110,9 @@ constexpr size_t kB1Bytes = sizeof(int32_t) * kBox * kBox;
 constexpr size_t kSgrBytes = kA0Bytes + kB0Bytes + kA1Bytes + kB1Bytes;
 constexpr size_t kHBytes = sizeof(int16_t) * kSRows * kMaxTile;
 constexpr size_t kRegion = kSgrBytes > kHBytes ? kSgrBytes : kHBytes;
-constexpr size_t kVBytes = sizeof(int32_t) * 2 * kVCols * kWarps;
-constexpr size_t kLrSmem = kSBytes + kRegion + 256 * sizeof(uint16_t) + kVBytes;
+constexpr size_t lr_smem(int threads) {
+    return kSBytes + kRegion + 256 * sizeof(uint16_t) + sizeof(int32_t) * 2 * kVCols * (threads / 32);
+}
 
 __device__ __forceinline__ int round2i(int v, int s) { return s == 0 ? v : (v + (1 << (s - 1))) >> s; }
 
@@ -171,12 +172,13 @@ __device__ __forceinline__ void box_ab(int sum, int sum_sq, int ar, int bc, uint
 // the columns those cover, bc < 64 - 2 RAD, as 2 RAD + 1 of them.  The last
 // few columns of every row (bc >= 64 - 2 RAD) are summed directly afterwards,
 // all rows' together, so no pass over a row runs with most lanes idle.
-template <int RAD>
+template <int RAD, int NT>
 __device__ __forceinline__ void box_pass(const uint16_t* __restrict__ S, uint16_t* __restrict__ A,
                                          int32_t* __restrict__ B, const uint16_t* __restrict__ a2tab,
                                          int32_t* __restrict__ V, int R, int C, int y_lo, bool odd_rows_only,
                                          const BoxConst& k) {
     constexpr int kMain = 64 - 2 * RAD;  // box columns the V buffer covers
+    constexpr int kWarps = NT / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rows = R + 2, cols = C + 2;
     const int main_cols = min(cols, kMain);
@@ -238,7 +240,7 @@ __device__ __forceinline__ void box_pass(const uint16_t* __restrict__ S, uint16_
     if (extra > 0) {
         const int nrows = odd_rows_only ? (rows + 1) >> 1 : rows;
         const unsigned mx = ((1u << 20) + extra - 1) / extra;  // i / extra = (i mx) >> 20 for i < 2^20 / extra
-        for (int i = threadIdx.x; i < nrows * extra; i += kLrThreads) {
+        for (int i = threadIdx.x; i < nrows * extra; i += NT) {
             const int row = (int)(((unsigned)i * mx) >> 20), bc = kMain + (i - row * extra);
             const int br = odd_rows_only ? 2 * row : row;
             const uint16_t* box = S + (br + 2 - RAD) * kSPitch + (kSOff - 1 - RAD) + bc;
@@ -257,7 +259,9 @@ __device__ __forceinline__ void box_pass(const uint16_t* __restrict__ S, uint16_
 }
 
 // One restoration tile: `block` indexes the tiles of all planes of `a`.
+template <int NT>
 __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
+    constexpr int kWarps = NT / 32, kRows = kMaxTile / kWarps;  // output rows of a warp
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* S = reinterpret_cast<uint16_t*>(smem_raw);
     unsigned char* region = smem_raw + kSBytes;
@@ -304,21 +308,22 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     if (P.copy_only || (u.type != VACO_AV1_LR_WIENER && u.type != VACO_AV1_LR_SGRPROJ)) {
         // RestorationUnit::None: the CDEF output, restoration.rs:194.  The
         // tile is at most 64 x 64 samples = 512 16-byte vectors, so each
-        // thread has both of its loads in flight before it stores.
+        // thread has all of its loads in flight before it stores.
         const bool vec = ((P.after.stride | P.out.stride) & 7) == 0 &&
                          ((reinterpret_cast<uintptr_t>(P.after.data) | reinterpret_cast<uintptr_t>(P.out.data)) & 15) == 0;
         const int vpr = (C + 7) >> 3;
         const unsigned mv = ((1u << 20) + vpr - 1) / vpr;  // i / vpr = (i mv) >> 20 for i < 2^20 / vpr
-        uint4 q[2];
+        constexpr int kLoads = 512 / NT;
+        uint4 q[kLoads];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = tid + j * kLrThreads, r = (int)(((unsigned)i * mv) >> 20), x = x_lo + 8 * (i - r * vpr);
+        for (int j = 0; j < kLoads; ++j) {
+            const int i = tid + j * NT, r = (int)(((unsigned)i * mv) >> 20), x = x_lo + 8 * (i - r * vpr);
             if (vec && i < R * vpr && x + 8 <= x_hi)
                 q[j] = __ldg(reinterpret_cast<const uint4*>(P.after.data + (long)(y_lo + r) * P.after.stride + x));
         }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = tid + j * kLrThreads, r = (int)(((unsigned)i * mv) >> 20), x = x_lo + 8 * (i - r * vpr);
+        for (int j = 0; j < kLoads; ++j) {
+            const int i = tid + j * NT, r = (int)(((unsigned)i * mv) >> 20), x = x_lo + 8 * (i - r * vpr);
             if (i >= R * vpr) continue;
             uint16_t* dst = P.out.data + (long)(y_lo + r) * P.out.stride + x;
             if (vec && x + 8 <= x_hi) {
@@ -341,7 +346,7 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     const DevPlaneC& BP = compact ? P.before_rows : P.before;
     const bool vec_ok = ((BP.stride | P.after.stride) & 7) == 0 &&
                         ((reinterpret_cast<uintptr_t>(BP.data) | reinterpret_cast<uintptr_t>(P.after.data)) & 15) == 0;
-    for (int i = tid; i < srows * (kSPitch / 8); i += kLrThreads) {
+    for (int i = tid; i < srows * (kSPitch / 8); i += NT) {
         const int r = i / (kSPitch / 8), v = i - r * (kSPitch / 8);
         const int y = clampi(y_lo - 3 + r, 0, P.height - 1);
         const uint16_t* row;
@@ -401,24 +406,24 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
             }
         }
         __syncthreads();
-        // Vertical pass: each thread walks rows 8 warp .. 8 warp + 7 of
-        // columns 2 lane and 2 lane + 1, reading each intermediate row once,
-        // both columns as one word.
-        const int k0 = 8 * warp;
+        // Vertical pass: each thread walks rows kRows warp .. kRows warp +
+        // kRows - 1 of columns 2 lane and 2 lane + 1, reading each intermediate
+        // row once, both columns as one word.
+        const int k0 = kRows * warp;
         const int c = 2 * lane;
         if (k0 >= R || c >= C) return;
         const bool second = c + 1 < C;
         const bool pair_store = ((P.out.stride | x_lo) & 1) == 0 && (reinterpret_cast<uintptr_t>(P.out.data) & 3) == 0;
-        int h[14][2];
+        int h[kRows + 6][2];
 #pragma unroll
-        for (int t = 0; t < 14; ++t) {
+        for (int t = 0; t < kRows + 6; ++t) {
             const uint32_t w = *reinterpret_cast<const uint32_t*>(H + min(k0 + t, kSRows - 1) * kMaxTile + c);
             h[t][0] = (int16_t)(w & 0xFFFF);
             h[t][1] = (int16_t)(w >> 16);
         }
         uint16_t* orow = P.out.data + (long)(y_lo + k0) * P.out.stride + x_lo + c;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < kRows; ++j) {
             if (k0 + j >= R) break;
             int v[2];
 #pragma unroll
@@ -450,17 +455,17 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     if (r0 != 0) {
         const SgrPassConst c = g_sgr_const.c[set][0];
         const BoxConst k{c.scale, c.p_lim, sh2, sh2 ? 1 << (sh2 - 1) : 0, sh1, sh1 ? 1 << (sh1 - 1) : 0};
-        box_pass<2>(S, A0, B0, a2tab, Vw, R, C, y_lo, true, k);
+        box_pass<2, NT>(S, A0, B0, a2tab, Vw, R, C, y_lo, true, k);
     }
     if (r1 != 0) {
         const SgrPassConst c = g_sgr_const.c[set][1];
         const BoxConst k{c.scale, c.p_lim, sh2, sh2 ? 1 << (sh2 - 1) : 0, sh1, sh1 ? 1 << (sh1 - 1) : 0};
-        box_pass<1>(S, A1, B1, a2tab, Vw, R, C, y_lo, false, k);
+        box_pass<1, NT>(S, A1, B1, a2tab, Vw, R, C, y_lo, false, k);
     }
     __syncthreads();
 
-    // Pixels of this thread: rows k0 .. k0+7 (k0 = 8 warp) of columns 2 lane
-    // and 2 lane + 1; pixel row k is box row k + 1.  Walking down its rows, a
+    // Pixels of this thread: rows k0 .. k0 + kRows - 1 (k0 = kRows warp, even) of
+    // columns 2 lane and 2 lane + 1; pixel row k is box row k + 1.  Walking down its rows, a
     // thread reads each box row of A / B once, the four box columns its two
     // pixels share as two 32-bit (A) and two 64-bit (B) loads.
     //   radius 2 (box rows of odd y only; y_lo is even, so pixel row k0 + j
@@ -471,7 +476,7 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     //   same three of the rows above and below, plus A[c] of those two --
     //   weight 4 on the cross, 3 on the corners.  Likewise for b.
     const int w0 = u.xqd[0], w1 = u.xqd[1];
-    const int k0 = 8 * warp;
+    const int k0 = kRows * warp;
     const int c = 2 * lane;
     if (k0 >= R || c >= C) return;
     const bool second = c + 1 < C;
@@ -514,7 +519,7 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     const bool pair_store = ((P.out.stride | x_lo) & 1) == 0 && (reinterpret_cast<uintptr_t>(P.out.data) & 3) == 0;
     uint16_t* orow = P.out.data + (long)(y_lo + k0) * P.out.stride + x_lo + c;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < kRows; ++j) {
         const int k = k0 + j;
         const uint32_t ow = *reinterpret_cast<const uint32_t*>(S + (k + 3) * kSPitch + kSOff + c);
         const int orig[2] = {(int)(ow & 0xFFFF), (int)(ow >> 16)};
@@ -559,9 +564,10 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     }
 }
 
-__global__ void __launch_bounds__(kLrThreads, 4) restoration_kernel(LrArgs a) {
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) restoration_kernel(LrArgs a) {
     overlap_prologue();
-    lr_tile(a, blockIdx.x);
+    lr_tile<NT>(a, blockIdx.x);
 }
 
 // Batched form: one CTA per tile of all frames of a batch (see dbcdef.cu).
@@ -572,7 +578,7 @@ __global__ void __launch_bounds__(kLrThreads, MIN_CTAS) restoration_batch_kernel
                                                                                 const int* __restrict__ tile_prefix,
                                                                                 int n) {
     const int f = frame_of_tile(tile_prefix, n, blockIdx.x);
-    lr_tile(frames[f], blockIdx.x - tile_prefix[f]);
+    lr_tile<kLrThreads>(frames[f], blockIdx.x - tile_prefix[f]);
 }
 
 // RestorationUnit::validate (restoration.rs:67-91).
@@ -654,28 +660,32 @@ cudaError_t lr_kernel_attributes() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !(g_lr_attr_devices.load(std::memory_order_acquire) & (1ull << dev))) {
-        cudaError_t e = cudaFuncSetAttribute(restoration_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kLrSmem);
+        const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        cudaError_t e = cudaFuncSetAttribute(restoration_kernel<kLrThreads>, attr, (int)lr_smem(kLrThreads));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(restoration_batch_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kLrSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(restoration_batch_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kLrSmem);
+            e = cudaFuncSetAttribute(restoration_kernel<kLrThreadsFew>, attr, (int)lr_smem(kLrThreadsFew));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(restoration_batch_kernel<3>, attr, (int)lr_smem(kLrThreads));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(restoration_batch_kernel<4>, attr, (int)lr_smem(kLrThreads));
         if (e != cudaSuccess) return e;
         g_lr_attr_devices.fetch_or(1ull << dev, std::memory_order_release);
     }
     return cudaSuccess;
 }
 
-cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, cudaStream_t stream) {
+cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, int sm_count, cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     LrArgs a;
     const int total = build_lr_args(planes, count, bit_depth, &a);
     cudaError_t e = lr_kernel_attributes();
     if (e != cudaSuccess) return e;
     if (total == 0) return cudaSuccess;
-    return launch_overlapped(restoration_kernel, dim3(total), dim3(kLrThreads), kLrSmem, stream, a);
+    // As in the fused kernel, tiles that are all resident at 512 threads (two
+    // CTAs per SM) take one tile's latency, which more warps shorten.
+    if (total <= 2 * sm_count)
+        return launch_overlapped(restoration_kernel<kLrThreadsFew>, dim3(total), dim3(kLrThreadsFew),
+                                 lr_smem(kLrThreadsFew), stream, a);
+    return launch_overlapped(restoration_kernel<kLrThreads>, dim3(total), dim3(kLrThreads), lr_smem(kLrThreads), stream,
+                             a);
 }
 
 cudaError_t launch_restoration_batch(const void* dev_args, const int* dev_prefix, int n, int tiles, int ctas_per_sm,
@@ -685,9 +695,9 @@ cudaError_t launch_restoration_batch(const void* dev_args, const int* dev_prefix
     if (e != cudaSuccess) return e;
     const LrArgs* args = static_cast<const LrArgs*>(dev_args);
     if (ctas_per_sm <= 3)
-        restoration_batch_kernel<3><<<tiles, kLrThreads, kLrSmem, stream>>>(args, dev_prefix, n);
+        restoration_batch_kernel<3><<<tiles, kLrThreads, lr_smem(kLrThreads), stream>>>(args, dev_prefix, n);
     else
-        restoration_batch_kernel<4><<<tiles, kLrThreads, kLrSmem, stream>>>(args, dev_prefix, n);
+        restoration_batch_kernel<4><<<tiles, kLrThreads, lr_smem(kLrThreads), stream>>>(args, dev_prefix, n);
     return cudaGetLastError();
 }
 
