@@ -219,6 +219,42 @@ const T* stage_array(vaco_av1_ctx* ctx, int slot, const T* host, size_t count, c
 
 // ---------------------------------------------------------------- stage runners (device pointers)
 
+// Whether the fused deblock+CDEF kernel takes this picture for one of its two
+// filters alone.  It needs the layouts AV1 can signal, Mi-padded extents of
+// whole 8x8 blocks, 32-bit output words, and, as its tiles read their
+// neighbours' input while those write, an output apart from the input.  Other
+// calls (in place, among them) take the per-stage kernels, which run in place.
+bool fused_takes(const vaco_av1_picture& src, const vaco_av1_picture& dst, const vaco_av1_frame_info& info) {
+    if (!bd_valid(info.bit_depth) || ((info.mi_cols | info.mi_rows) & 1)) return false;
+    const int np = info.monochrome ? 1 : 3;
+    if (np > 1 && !av1_subsampling_ok(info.subsampling_x, info.subsampling_y)) return false;
+    auto range = [](const vaco_av1_picture& p, int k, uintptr_t* lo, uintptr_t* hi) {
+        *lo = reinterpret_cast<uintptr_t>(p.planes[k]);
+        *hi = *lo + 2 * ((size_t)p.stride[k] * (p.height[k] - 1) + p.width[k]);
+    };
+    for (int k = 0; k < np; ++k) {
+        if ((dst.stride[k] & 1) || (reinterpret_cast<uintptr_t>(dst.planes[k]) & 3)) return false;
+        uintptr_t d0, d1;
+        range(dst, k, &d0, &d1);
+        for (int j = 0; j < np; ++j) {
+            uintptr_t s0, s1;
+            range(src, j, &s0, &s1);
+            if (d0 < s1 && s0 < d1) return false;
+        }
+    }
+    return true;
+}
+
+// The fused kernel as one filter alone: `L` has the pictures and that filter's
+// parameters.
+cudaError_t run_fused(vaco_av1_ctx* ctx, cudaStream_t s, DbCdefLaunch& L) {
+    for (DevPlane& r : L.pre_rows) r = DevPlane{nullptr, 0, 0, 0};
+    L.status = ctx->status;
+    L.sm_count = ctx->sm_count;
+    ctx->launches++;
+    return launch_dbcdef(L, s);
+}
+
 // Deblocking: src -> dst (copy + checks + both passes).  Returns host key.
 unsigned long long run_deblock(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_picture& src,
                                const vaco_av1_picture& dst, const vaco_av1_frame_info& info, const uint8_t* tx_luma,
@@ -229,6 +265,20 @@ unsigned long long run_deblock(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1
     for (int k = 0; k < 4; ++k) params_ok = params_ok && params.levels[k] <= 63;
     if (!params_ok || !tx_luma || (np > 1 && !tx_chroma)) {
         return make_key(STAGE_DEBLOCK, 0, params_ok ? VACO_AV1_MSG_NULL_ARGUMENT : VACO_AV1_MSG_DB_PARAMS);
+    }
+    if (fused_takes(src, dst, info)) {
+        // one pass over the picture instead of a check, a copy per plane and
+        // two filter passes: 1080p 10-bit 4:2:0 43 -> 18 us of kernels
+        DbCdefLaunch L{};
+        L.src = src;
+        L.dst = dst;
+        L.info = info;
+        L.tx_luma = tx_luma;
+        L.tx_chroma = tx_chroma;
+        L.lvl_map = lvl_map;
+        L.deblock = params;
+        *err = run_fused(ctx, s, L);
+        return kNoError;
     }
     DevPlaneC sp[3];
     DevPlane dp[3];
@@ -515,6 +565,31 @@ int32_t vaco_av1_cdef_picture_dev(vaco_av1_ctx* ctx, void* stream, const vaco_av
     cudaSetDevice(ctx->device);
     cudaError_t e = reset_status(ctx, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+    bool all_zero = true;
+    for (int k = 0; k < 8; ++k)
+        all_zero = all_zero && params->y_primary[k] == 0 && params->y_secondary[k] == 0 && params->uv_primary[k] == 0 &&
+                   params->uv_secondary[k] == 0;
+    if (params->enabled && !all_zero && skip && (cdef_idx || cdef_count <= 0) && fused_takes(*src, *dst, *info)) {
+        // The fused kernel with deblocking off.  It checks more than
+        // apply_cdef does (every sample, where vaco looks at the filtered
+        // blocks alone) and names the error less closely, so a picture that
+        // it objects to goes to the per-stage kernel below, whose word counts.
+        DbCdefLaunch L{};
+        L.src = *src;
+        L.dst = *dst;
+        L.info = *info;
+        L.skip = skip;
+        L.cdef_idx = cdef_idx;
+        L.cdef_stride = cdef_stride;
+        L.cdef_count = cdef_count;
+        L.cdef = *params;
+        e = run_fused(ctx, s, L);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+        const int32_t st = finish(ctx, s, kNoError, msg);
+        if (st != VACO_AV1_INVALID_DATA) return st;
+        e = reset_status(ctx, s);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+    }
     unsigned long long hk = run_cdef(ctx, s, *src, *dst, *info, skip, cdef_idx, cdef_stride, cdef_count, *params, &e);
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
     return finish(ctx, s, hk, msg);
@@ -726,20 +801,13 @@ int32_t vaco_av1_restore_plane_dev(vaco_av1_ctx* ctx, void* stream, const uint16
     cudaStream_t s = (cudaStream_t)stream;
     cudaSetDevice(ctx->device);
     cudaError_t e = reset_status(ctx, s);
-    if (e == cudaSuccess) e = launch_lr_unit_check(units, unit_count, 0, ctx->status, s);
-    const int maxv = (1 << config->bit_depth) - 1;
+    // The checks must pass before filtering (restore_plane validates first):
+    // the filter's tiles do nothing once the status word holds an error.
     if (e == cudaSuccess)
-        e = launch_range_check(DevPlaneC{before, before_width, before_height, before_stride}, config->width,
-                               config->height, maxv, ctx->status, STAGE_LR, lr_position(0, LR_SAMPLE, 0),
-                               VACO_AV1_MSG_LR_SAMPLE, s);
-    if (e == cudaSuccess)
-        e = launch_range_check(DevPlaneC{after, after_width, after_height, after_stride}, config->width,
-                               config->height, maxv, ctx->status, STAGE_LR, lr_position(0, LR_SAMPLE, 0),
-                               VACO_AV1_MSG_LR_SAMPLE, s);
-    // The checks must pass before filtering: restore_plane validates first.
-    int32_t st = e == cudaSuccess ? finish(ctx, s, kNoError, msg) : cuda_fail(ctx, e, msg);
-    ctx->launches += 3;
-    if (st != VACO_AV1_OK) return st;
+        e = launch_lr_check(units, unit_count, DevPlaneC{before, before_width, before_height, before_stride},
+                            DevPlaneC{after, after_width, after_height, after_stride}, config->width, config->height,
+                            config->bit_depth, ctx->sm_count, ctx->status, s);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
     LrPlane p;
     p.before = DevPlaneC{before, before_width, before_height, before_stride};
     p.before_rows = DevPlaneC{nullptr, 0, 0, 0};
@@ -755,12 +823,10 @@ int32_t vaco_av1_restore_plane_dev(vaco_av1_ctx* ctx, void* stream, const uint16
     p.copy_only = 0;
     p.plane_index = 0;
     p.unit_status = nullptr;  // validated by the checks above
-    e = launch_restoration(&p, 1, config->bit_depth, ctx->sm_count, s);
-    ctx->launches++;
+    e = launch_restoration(&p, 1, config->bit_depth, ctx->sm_count, s, ctx->status);
+    ctx->launches += 2;
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
-    e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
-    return set_msg(msg, VACO_AV1_MSG_NONE), VACO_AV1_OK;
+    return finish(ctx, s, kNoError, msg);
 }
 
 int32_t vaco_av1_restore_plane_host(vaco_av1_ctx* ctx, const uint16_t* before, int32_t before_width,

@@ -112,6 +112,7 @@ struct DbCdefArgs {
     uint8_t y_pri[8], y_sec[8], uv_pri[8], uv_sec[8];
     DeviceStatus* status;
     int vec_ok;
+    int dst_vec;                // the CDEF planes' rows start 16-byte aligned
     int staged_vectors;         // 16-byte vectors of all staged planes together
     DirectPlane direct[3];      // final output written here too (see DirectPlane)
     size_t plane_off[3];        // shared-memory offset (samples) of each staged plane
@@ -487,7 +488,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     // copies are in flight (cells the two passes touch; see SideWindow).  Each
     // cell is checked where it is loaded: the windows of all tiles together
     // hold exactly the maps' cells.
-    {
+    if (a.tx_luma) {  // null for CDEF alone
         const int crows = (a.mi_rows + ssy) >> ssy, ccols = (a.mi_cols + ssx) >> ssx;
         const int cr0 = (mi_r0 >> ssy) - kWinTop, cc0 = (mi_c0 >> ssx) - kWinLeft;
         int bad = 0;
@@ -577,6 +578,16 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
             const int px0 = x0 >> g.sx, py0 = y0 >> g.sy;
             const DirectPlane* D = DIRECT ? &a.direct[p] : nullptr;
             const uint16_t* t = smem + a.plane_off[p];
+            if (a.dst_vec && !(D && D->out.data) && px0 + g.tw <= d.width) {  // whole rows of 16-byte vectors
+                const int lv = 3 - g.sx;  // log2 of the vectors of a row
+                for (int i = tid; i < g.th << lv; i += NT) {
+                    const int r = i >> lv, c = (i & ((1 << lv) - 1)) * 8, y = py0 + r;
+                    if (y >= d.height) break;
+                    *reinterpret_cast<uint4*>(d.data + (long)y * d.stride + px0 + c) =
+                        *reinterpret_cast<const uint4*>(t + (r + kHalo) * g.pitch + kHalo + c);
+                }
+                continue;
+            }
             for (int r = warp; r < g.th; r += kWarpsNT) {
                 const int y = py0 + r;
                 if (y >= d.height) break;
@@ -750,7 +761,7 @@ size_t build_dbcdef_args(const DbCdefLaunch& L, void* out) {
     DbCdefArgs a;
     memset(&a, 0, sizeof a);
     const int np = L.info.monochrome ? 1 : 3;
-    bool vec = true;
+    bool vec = true, dst_vec = true;
     size_t off = 0;
     for (int p = 0; p < 3; ++p) {
         a.src[p] = DevPlaneC{L.src.planes[p], L.src.width[p], L.src.height[p], L.src.stride[p]};
@@ -759,6 +770,7 @@ size_t build_dbcdef_args(const DbCdefLaunch& L, void* out) {
         a.plane_off[p] = off;
         if (p < np) {
             vec = vec && (L.src.stride[p] % 8 == 0) && ((uintptr_t)L.src.planes[p] % 16 == 0);
+            dst_vec = dst_vec && (L.dst.stride[p] % 8 == 0) && ((uintptr_t)L.dst.planes[p] % 16 == 0);
             const int sx = p ? L.info.subsampling_x : 0, sy = p ? L.info.subsampling_y : 0;
             off += (size_t)((64 >> sx) + 2 * kHalo) * ((64 >> sy) + 2 * kHalo);
         }
@@ -796,6 +808,7 @@ size_t build_dbcdef_args(const DbCdefLaunch& L, void* out) {
     }
     a.status = L.status;
     a.vec_ok = vec;
+    a.dst_vec = dst_vec;
     a.staged_vectors = (int)(off / 8);  // each staged plane is a multiple of 8 samples
     for (int p = 0; p < 3; ++p) a.direct[p] = p < np ? L.direct[p] : DirectPlane{};
     memcpy(out, &a, sizeof a);

