@@ -402,12 +402,11 @@ VACO_AV1_API int32_t vaco_av1_postfilter_frame_host(vaco_av1_ctx* ctx, const vac
 /* Launch-shape knobs for the batched form (no counterpart in vaco).  The
  * values in tuned/ are picked by vaco_b200.autotune on the target GPU. */
 typedef struct vaco_av1_tuning {
-    int32_t dbcdef_ctas_per_sm;  /* resident CTAs per SM the batched deblock+CDEF kernel
-                                    is compiled for, i.e. its register budget (1..8):
-                                    up to 3 -> 80 registers a thread, 4 and more -> 64
-                                    (256-thread tiles; 128-thread tiles have one body) */
-    int32_t lr_ctas_per_sm;      /* the same for the batched restoration kernel (1..8):
-                                    up to 3 -> 80 registers, 4 and more -> 64 */
+    int32_t dbcdef_ctas_per_sm;  /* 1..8; without effect: the batched deblock+CDEF kernel
+                                    has one register budget per threads a tile */
+    int32_t lr_ctas_per_sm;      /* resident CTAs per SM the batched restoration kernel is
+                                    compiled for, i.e. its register budget (1..8): up to
+                                    3 -> 80 registers a thread, 4 and more -> 64 */
     int32_t use_graphs;          /* capture each batch composition once as a CUDA graph */
     int32_t largest_first;       /* lay the largest frames' tiles first in the launch */
     int32_t dbcdef_threads;      /* threads per 64x64 tile of the deblock+CDEF kernel, in the

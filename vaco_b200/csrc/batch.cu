@@ -453,8 +453,8 @@ int32_t vaco::batch_enqueue(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_fr
         }
         if (r == cudaSuccess && fused && !order.empty() && db_prefix[order.size()] > 0)
             r = launch_dbcdef_batch(dtab + off_db, reinterpret_cast<const int*>(dtab + off_db_prefix), (int)order.size(),
-                                    db_prefix[order.size()], smem_db, ctx->tuning.dbcdef_ctas_per_sm,
-                                    ctx->tuning.dbcdef_threads, layout, max_depth, s);
+                                    db_prefix[order.size()], smem_db, ctx->tuning.dbcdef_threads, layout, max_depth,
+                                    s);
         for (int i : order) {
             const FramePlan& F = plan[i];
             if (r != cudaSuccess || !F.superres) continue;

@@ -725,7 +725,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
 // as 3 (80 registers) on 1080p and on 2560-, 2880- and 3840-wide frames
 // (1.5-2 % faster on the last two); 128 threads at 5 CTAs
 // per SM is the smaller-CTA shape (shorter barriers, about the same warps per
-// SM).  The batched form also has the 256 x 3 body (see dbcdef_batch_kernel).
+// SM).
 // DIRECT: a body that also writes the output of planes without restoration
 // (DirectPlane); the code for it measured 3 % slower on frames that have no
 // such plane, so it is a separate body.
@@ -745,6 +745,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_kernel(DbCdefArgs a) {
 template <int NT, int MIN_CTAS, int LAYOUT, class Block>
 __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_batch_kernel(const DbCdefArgs* __restrict__ frames,
                                                                     const int* __restrict__ tile_prefix, int n) {
+    overlap_prologue();
     const int f = frame_of_tile(tile_prefix, n, blockIdx.x);
     const DbCdefArgs& a = frames[f];
     const int local = blockIdx.x - tile_prefix[f];
@@ -835,9 +836,9 @@ cudaError_t dbcdef_kernel_attributes() {
                            dbcdef_kernel<512, 2, 3, B>, dbcdef_kernel<512, 2, 0, B, true>,
                            dbcdef_kernel<512, 2, 1, B, true>, dbcdef_kernel<512, 2, 3, B, true>})
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(k, attr, kMaxSmem);
-            for (auto k : {dbcdef_batch_kernel<256, 3, -1, B>, dbcdef_batch_kernel<256, 3, 0, B>,
-                           dbcdef_batch_kernel<256, 3, 1, B>, dbcdef_batch_kernel<256, 3, 3, B>,
-                           dbcdef_batch_kernel<256, 4, -1, B>, dbcdef_batch_kernel<128, 5, -1, B>})
+            for (auto k : {dbcdef_batch_kernel<256, 4, 0, B>, dbcdef_batch_kernel<256, 4, 1, B>,
+                           dbcdef_batch_kernel<256, 4, 3, B>, dbcdef_batch_kernel<256, 4, -1, B>,
+                           dbcdef_batch_kernel<128, 5, -1, B>})
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(k, attr, kMaxSmem);
         };
         optin(HalfBlock{});
@@ -890,31 +891,27 @@ cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream) {
 
 template <class Block>
 static cudaError_t launch_dbcdef_batch_as(const DbCdefArgs* args, const int* dev_prefix, int n, int tiles, size_t smem,
-                                          int ctas_per_sm, int threads, int layout, cudaStream_t stream) {
+                                          int threads, int layout, cudaStream_t stream) {
     using K = void (*)(const DbCdefArgs*, const int*, int);
     K k;
     if (threads == 128) {
         k = dbcdef_batch_kernel<128, 5, -1, Block>;
-    } else if (ctas_per_sm <= 3) {  // up to 3 resident: the 80-register body
-        k = layout == 3 ? dbcdef_batch_kernel<256, 3, 3, Block> : layout == 1 ? dbcdef_batch_kernel<256, 3, 1, Block>
-          : layout == 0 ? dbcdef_batch_kernel<256, 3, 0, Block> : dbcdef_batch_kernel<256, 3, -1, Block>;
-    } else {  // 64 registers: the layout-specialised bodies would spill
-        k = dbcdef_batch_kernel<256, 4, -1, Block>;
+    } else {  // as the per-frame kernel; at 3 CTAs per SM (80 registers) the mix of frames is 4.5 % slower
+        k = layout == 3 ? dbcdef_batch_kernel<256, 4, 3, Block> : layout == 1 ? dbcdef_batch_kernel<256, 4, 1, Block>
+          : layout == 0 ? dbcdef_batch_kernel<256, 4, 0, Block> : dbcdef_batch_kernel<256, 4, -1, Block>;
     }
-    k<<<tiles, threads == 128 ? 128 : 256, smem, stream>>>(args, dev_prefix, n);
-    return cudaGetLastError();
+    return launch_overlapped(k, dim3(tiles), dim3(threads == 128 ? 128 : 256), smem, stream, args, dev_prefix, n);
 }
 
 cudaError_t launch_dbcdef_batch(const void* dev_args, const int* dev_prefix, int n, int tiles, size_t smem,
-                                int ctas_per_sm, int threads, int layout, int max_bit_depth, cudaStream_t stream) {
+                                int threads, int layout, int max_bit_depth, cudaStream_t stream) {
     if (tiles <= 0) return cudaSuccess;
     cudaError_t e = dbcdef_kernel_attributes();
     if (e != cudaSuccess) return e;
     const DbCdefArgs* args = static_cast<const DbCdefArgs*>(dev_args);
     return max_bit_depth <= 10
-               ? launch_dbcdef_batch_as<HalfBlock>(args, dev_prefix, n, tiles, smem, ctas_per_sm, threads, layout, stream)
-               : launch_dbcdef_batch_as<PairBlock>(args, dev_prefix, n, tiles, smem, ctas_per_sm, threads, layout,
-                                                   stream);
+               ? launch_dbcdef_batch_as<HalfBlock>(args, dev_prefix, n, tiles, smem, threads, layout, stream)
+               : launch_dbcdef_batch_as<PairBlock>(args, dev_prefix, n, tiles, smem, threads, layout, stream);
 }
 
 }  // namespace vaco

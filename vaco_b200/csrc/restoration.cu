@@ -579,6 +579,7 @@ template <int MIN_CTAS>
 __global__ void __launch_bounds__(kLrThreads, MIN_CTAS) restoration_batch_kernel(const LrArgs* __restrict__ frames,
                                                                                 const int* __restrict__ tile_prefix,
                                                                                 int n) {
+    overlap_prologue();
     const int f = frame_of_tile(tile_prefix, n, blockIdx.x);
     lr_tile<kLrThreads>(frames[f], blockIdx.x - tile_prefix[f]);
 }
@@ -726,11 +727,8 @@ cudaError_t launch_restoration_batch(const void* dev_args, const int* dev_prefix
     cudaError_t e = lr_kernel_attributes();
     if (e != cudaSuccess) return e;
     const LrArgs* args = static_cast<const LrArgs*>(dev_args);
-    if (ctas_per_sm <= 3)
-        restoration_batch_kernel<3><<<tiles, kLrThreads, lr_smem(kLrThreads), stream>>>(args, dev_prefix, n);
-    else
-        restoration_batch_kernel<4><<<tiles, kLrThreads, lr_smem(kLrThreads), stream>>>(args, dev_prefix, n);
-    return cudaGetLastError();
+    return launch_overlapped(ctas_per_sm <= 3 ? restoration_batch_kernel<3> : restoration_batch_kernel<4>, dim3(tiles),
+                             dim3(kLrThreads), lr_smem(kLrThreads), stream, args, dev_prefix, n);
 }
 
 cudaError_t launch_lr_unit_check(const vaco_av1_lr_unit* units, int n, int plane, DeviceStatus* status,
