@@ -133,15 +133,7 @@ __device__ __forceinline__ bool unit_ok(const vaco_av1_lr_unit& u) {
 }
 
 
-// Box sums around every box position (br, bc) -- box rows y_lo-1+br (only
-// those of odd y when odd_rows_only), box columns x_lo-1+bc -- and the a2 / b
-// terms of box_ab (restoration.rs:314-339).  A warp takes whole box rows:
-// its lanes first form the (2 RAD + 1)-row vertical sums (and sums of
-// squares) of every column the row's boxes reach, in the warp's own buffer
-// V, then each box sum as 2 RAD + 1 of those -- 2 (2 RAD + 1) loads per box
-// instead of (2 RAD + 1)^2.
-// box_ab's a2 and b (restoration.rs:314-339) from a box sum and sum of
-// squares, stored at box position (ar, bc).
+// box_ab's a2 and b (restoration.rs:314-339) from a box sum and sum of squares.
 // A pass's constants for box_ab: scale and p_lim of its set, and the
 // Round2 shifts by 2 (bd - 8) and bd - 8 as (v + half) >> shift.
 struct BoxConst {
@@ -150,19 +142,16 @@ struct BoxConst {
 };
 
 template <int RAD>
-__device__ __forceinline__ void box_ab(int sum, int sum_sq, int ar, int bc, uint16_t* __restrict__ A,
-                                       int32_t* __restrict__ B, const uint16_t* __restrict__ a2tab,
-                                       const BoxConst& k) {
+__device__ __forceinline__ void box_ab(int sum, int sum_sq, const uint16_t* __restrict__ a2tab, const BoxConst& k,
+                                       unsigned& a2, int& b) {
     constexpr int n = (2 * RAD + 1) * (2 * RAD + 1);
     constexpr unsigned recip = ((1 << 12) + n / 2) / n;
     const int aa = (sum_sq + k.half_sq) >> k.sh_sq;
     const int d = (sum + k.half) >> k.sh;
     const unsigned p = (unsigned)max(aa * n - d * d, 0);
     const unsigned z = min((min(p, k.p_lim) * k.scale + (1u << 19)) >> 20, 255u);
-    const int a2 = a2tab[z];
-    const unsigned b = ((unsigned)(256 - a2) * (unsigned)sum * recip + (1u << 11)) >> 12;
-    A[ar * kBox + bc] = (uint16_t)a2;
-    B[ar * kBox + bc] = (int)b;
+    a2 = a2tab[z];
+    b = (int)(((256u - a2) * recip * (unsigned)sum + (1u << 11)) >> 12);
 }
 
 // Box sums around every box position (br, bc) -- box rows y_lo-1+br (only
@@ -228,11 +217,16 @@ __device__ __forceinline__ void box_pass(const uint16_t* __restrict__ S, uint16_
                     sum += vs[dx];
                     sum_sq += vq[dx];
                 }
-                const int ar = odd_rows_only ? br >> 1 : br;
-                box_ab<RAD>(sum, sum_sq, ar, bc, A, B, a2tab, k);
-                if (bc + 1 < main_cols)
-                    box_ab<RAD>(sum - vs[0] + vs[2 * RAD + 1], sum_sq - vq[0] + vq[2 * RAD + 1], ar, bc + 1, A, B,
-                                a2tab, k);
+                // both boxes' terms as one word and one 64-bit word (an odd
+                // count writes one position more, which nothing reads before
+                // the remaining columns below are written)
+                const int at = (odd_rows_only ? br >> 1 : br) * kBox + bc;
+                unsigned a0, a1;
+                int b0, b1;
+                box_ab<RAD>(sum, sum_sq, a2tab, k, a0, b0);
+                box_ab<RAD>(sum - vs[0] + vs[2 * RAD + 1], sum_sq - vq[0] + vq[2 * RAD + 1], a2tab, k, a1, b1);
+                *reinterpret_cast<uint32_t*>(A + at) = a0 | a1 << 16;
+                *reinterpret_cast<int2*>(B + at) = make_int2(b0, b1);
             }
         }
     }
@@ -254,7 +248,11 @@ __device__ __forceinline__ void box_pass(const uint16_t* __restrict__ S, uint16_
                     sum += v;
                     sum_sq += v * v;
                 }
-            box_ab<RAD>(sum, sum_sq, row, bc, A, B, a2tab, k);
+            unsigned a2;
+            int b;
+            box_ab<RAD>(sum, sum_sq, a2tab, k, a2, b);
+            A[row * kBox + bc] = (uint16_t)a2;
+            B[row * kBox + bc] = b;
         }
     }
 }
@@ -481,34 +479,41 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     const int c = 2 * lane;
     if (k0 >= R || c >= C) return;
     const bool second = c + 1 < C;
-    // box columns c .. c + 3 of a row (the neighbourhoods of pixels c, c + 1)
-    auto quad = [&](const uint16_t* A, const int32_t* B, int i, int (&qa)[4], int (&qb)[4]) {
-        const uint32_t a01 = *reinterpret_cast<const uint32_t*>(A + i);
-        const uint32_t a23 = *reinterpret_cast<const uint32_t*>(A + i + 2);
-        const int2 b01 = *reinterpret_cast<const int2*>(B + i);
-        const int2 b23 = *reinterpret_cast<const int2*>(B + i + 2);
-        qa[0] = a01 & 0xFFFF, qa[1] = a01 >> 16, qa[2] = a23 & 0xFFFF, qa[3] = a23 >> 16;
-        qb[0] = b01.x, qb[1] = b01.y, qb[2] = b23.x, qb[3] = b23.y;
+    // Weighted sums of box columns c .. c + 2 (pixel c) and c + 1 .. c + 3 (pixel
+    // c + 1) of a row.  A's four columns come as two words of two, which dp2a
+    // weighs as they are; B's weights are multiples of the plain sum plus one
+    // more middle column.
+    auto weigh_a = [&](const uint16_t* A, int i, unsigned outer, unsigned mid, int (&g)[2]) {
+        const uint32_t q01 = *reinterpret_cast<const uint32_t*>(A + i), q23 = *reinterpret_cast<const uint32_t*>(A + i + 2);
+        g[0] = (int)__dp2a_lo(q23, outer, __dp2a_lo(q01, outer | mid << 8, 0u));
+        g[1] = (int)__dp2a_lo(q23, mid | outer << 8, __dp2a_lo(q01, outer << 8, 0u));
+    };
+    struct Sum3 {
+        int s[2], mid[2];
+    };
+    auto sum_b = [&](const int32_t* B, int i) {
+        const int2 b01 = *reinterpret_cast<const int2*>(B + i), b23 = *reinterpret_cast<const int2*>(B + i + 2);
+        return Sum3{{b01.x + b01.y + b23.x, b01.y + b23.x + b23.y}, {b01.y, b23.x}};
     };
     auto g0 = [&](int br, int (&ga)[2], int (&gb)[2]) {  // br even: compact row br / 2
-        int qa[4], qb[4];
-        quad(A0, B0, (br >> 1) * kBox + c, qa, qb);
+        const int i = (br >> 1) * kBox + c;
+        weigh_a(A0, i, 5, 6, ga);
+        const Sum3 t = sum_b(B0, i);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            ga[x] = 5 * (qa[x] + qa[x + 2]) + 6 * qa[x + 1];
-            gb[x] = 5 * (qb[x] + qb[x + 2]) + 6 * qb[x + 1];
-        }
+        for (int x = 0; x < 2; ++x) gb[x] = 5 * t.s[x] + t.mid[x];
     };
-    int h3a[3][2], h3b[3][2], ca[3][2], cb[3][2];
+    // As the row itself (cross weights, with the Round2 term of f1) and as a
+    // neighbour of the row above or below.
+    int own_a[3][2], own_b[3][2], next_a[3][2], next_b[3][2];
     auto row1 = [&](int br, int slot) {
-        int qa[4], qb[4];
-        quad(A1, B1, br * kBox + c, qa, qb);
+        const int i = br * kBox + c;
+        weigh_a(A1, i, 4, 4, own_a[slot]);
+        weigh_a(A1, i, 3, 4, next_a[slot]);
+        const Sum3 t = sum_b(B1, i);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-            ca[slot][x] = qa[x + 1];
-            cb[slot][x] = qb[x + 1];
-            h3a[slot][x] = qa[x] + qa[x + 1] + qa[x + 2];
-            h3b[slot][x] = qb[x] + qb[x + 1] + qb[x + 2];
+            own_b[slot][x] = 4 * t.s[x] + 256;
+            next_b[slot][x] = 3 * t.s[x] + t.mid[x];
         }
     };
     int pa[2] = {0, 0}, pb[2] = {0, 0}, na[2] = {0, 0}, nb[2] = {0, 0};
@@ -519,6 +524,7 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     }
     const bool pair_store = ((P.out.stride | x_lo) & 1) == 0 && (reinterpret_cast<uintptr_t>(P.out.data) & 3) == 0;
     uint16_t* orow = P.out.data + (long)(y_lo + k0) * P.out.stride + x_lo + c;
+    const int w1s = w1 << 4, w2 = 128 - w0 - w1;
 #pragma unroll
     for (int j = 0; j < kRows; ++j) {
         const int k = k0 + j;
@@ -529,11 +535,11 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
             if ((j & 1) == 0) {
                 g0(k + 2, na, nb);
 #pragma unroll
-                for (int x = 0; x < 2; ++x) f0[x] = round2i((pa[x] + na[x]) * orig[x] + (pb[x] + nb[x]), 9);
+                for (int x = 0; x < 2; ++x) f0[x] = ((pa[x] + na[x]) * orig[x] + (pb[x] + nb[x] + 256)) >> 9;
             } else {
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    f0[x] = round2i(na[x] * orig[x] + nb[x], 8);
+                    f0[x] = (na[x] * orig[x] + (nb[x] + 128)) >> 8;
                     pa[x] = na[x];
                     pb[x] = nb[x];
                 }
@@ -544,16 +550,16 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
             const int u_ = j % 3, m_ = (j + 1) % 3, d_ = (j + 2) % 3;
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                const int aa = 4 * h3a[m_][x] + 3 * (h3a[u_][x] + h3a[d_][x]) + ca[u_][x] + ca[d_][x];
-                const int bb = 4 * h3b[m_][x] + 3 * (h3b[u_][x] + h3b[d_][x]) + cb[u_][x] + cb[d_][x];
-                f1[x] = round2i(aa * orig[x] + bb, 9);
+                const int aa = own_a[m_][x] + next_a[u_][x] + next_a[d_][x];
+                const int bb = own_b[m_][x] + next_b[u_][x] + next_b[d_][x];
+                f1[x] = (aa * orig[x] + bb) >> 9;
             }
         }
         if (k < R) {
             int v[2];
 #pragma unroll
             for (int x = 0; x < 2; ++x)
-                v[x] = clampi(round2i(w0 * f0[x] + w1 * (orig[x] << 4) + (128 - w0 - w1) * f1[x], 11), 0, maxv);
+                v[x] = __vimin_s32_relu((w0 * f0[x] + (w1s * orig[x] + 1024) + w2 * f1[x]) >> 11, maxv);
             if (pair_store && second) {
                 *reinterpret_cast<uint32_t*>(orow) = (uint32_t)v[0] | ((uint32_t)v[1] << 16);
             } else {
