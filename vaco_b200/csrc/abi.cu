@@ -403,6 +403,10 @@ void vaco_av1_ctx_destroy(vaco_av1_ctx* ctx) {
         if (slot.status) cudaFree(slot.status);
         if (slot.status_host) cudaFreeHost(slot.status_host);
     }
+    for (int k = 0; k < vaco_av1_ctx::kMaxBands; ++k)
+        for (cudaEvent_t ev : {ctx->band_staged[k], ctx->band_filtered[k]})
+            if (ev) cudaEventDestroy(ev);
+    if (ctx->side_host) cudaFreeHost(ctx->side_host);
     for (auto& g : ctx->grain) {
         if (g.stream) cudaStreamSynchronize(g.stream);
         for (cudaEvent_t ev : {g.ready, g.free})
@@ -941,11 +945,23 @@ static bool chain_geometry_ok(const vaco_av1_frame_job* j, bool check_dst = true
     return true;
 }
 
+// The kernels of a chain without superres, for a caller that launches them a
+// band of rows at a time.
+struct ChainKernels {
+    DbCdefLaunch db;
+    bool run_db = false;
+    LrPlane lr[3];
+    int nlr = 0;
+    DirectPlane direct[3];
+    unsigned long long host_key = kNoError;
+};
+
 // The chain on device pointers.  Deblocking and CDEF run fused
 // (dbcdef.cu): the deblocked picture exists only as restoration's compact
-// stripe-boundary rows.
+// stripe-boundary rows.  With `later`, nothing is launched or waited for: the
+// kernels go there (no superres).
 static int32_t postfilter_dev_impl(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_frame_job* job, int32_t* msg,
-                                   bool defer) {
+                                   bool defer, ChainKernels* later = nullptr) {
     const vaco_av1_frame_info& info = job->info;
     const int np = info.monochrome ? 1 : 3;
     const int ssx = info.subsampling_x, ssy = info.subsampling_y;
@@ -1020,9 +1036,15 @@ static int32_t postfilter_dev_impl(vaco_av1_ctx* ctx, cudaStream_t s, const vaco
             L.threads = ctx->tuning.dbcdef_threads == 128 ? 128 : 256;
             L.sm_count = ctx->sm_count;
             for (int k = 0; k < 3; ++k) L.direct[k] = direct[k];
-            e = launch_dbcdef(L, s);
-            ctx->launches++;
-            if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+            if (later) {
+                later->db = L;
+                later->run_db = true;
+                for (int k = 0; k < 3; ++k) later->direct[k] = direct[k];
+            } else {
+                e = launch_dbcdef(L, s);
+                ctx->launches++;
+                if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+            }
         }
     }
     ctx->mark(1, s);
@@ -1123,11 +1145,18 @@ static int32_t postfilter_dev_impl(vaco_av1_ctx* ctx, cudaStream_t s, const vaco
         // Samples reaching restoration inside the chain were produced by the
         // deblocking / CDEF / superres kernels from range-checked input, so
         // they are in range by construction: no second scan is needed.
-        if (hk == kNoError && nlr > 0) {
+        if (later && hk == kNoError) {
+            for (int k = 0; k < nlr; ++k) later->lr[k] = lp[k];
+            later->nlr = nlr;
+        } else if (hk == kNoError && nlr > 0) {
             e = launch_restoration(lp, nlr, info.bit_depth, ctx->sm_count, s);
             ctx->launches++;
             if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
         }
+    }
+    if (later) {
+        later->host_key = hk;
+        return VACO_AV1_OK;
     }
     ctx->mark(4, s);
     if (defer) {
@@ -1149,22 +1178,13 @@ int32_t vaco_av1_postfilter_frame_dev(vaco_av1_ctx* ctx, void* stream, const vac
     return postfilter_dev_impl(ctx, (cudaStream_t)stream, job, msg, ctx->deferred);
 }
 
-// The chain on a job whose pictures and side information are in host memory:
-// stages the inputs into context scratch, runs the chain into a device
-// picture `*d_out` (context scratch), and leaves the stream synchronized.
-// With sc != s the inputs are copied on stream sc, which `staged` then
-// orders before the chain on s; `defer` is postfilter_dev_impl's.
-static int32_t postfilter_from_host(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_frame_job* job,
-                                    vaco_av1_picture* d_out, int32_t* msg, cudaStream_t sc = nullptr,
-                                    cudaEvent_t staged = nullptr, bool defer = false) {
-    if (!sc) sc = s;
+// Copies a host job's side information to context scratch on stream sc and
+// points the device job `d` at it.
+static cudaError_t stage_side(vaco_av1_ctx* ctx, const vaco_av1_frame_job* job, vaco_av1_frame_job& d, cudaStream_t sc) {
     const vaco_av1_frame_info& info = job->info;
     const int np = info.monochrome ? 1 : 3;
     const int ssx = info.subsampling_x, ssy = info.subsampling_y;
     cudaError_t e = cudaSuccess;
-    vaco_av1_frame_job d = *job;
-    if (!stage_picture_in(ctx, &job->src, np, S_H_IN0, &d.src, sc, &e)) return cuda_fail(ctx, e, msg);
-    if (!alloc_picture(ctx, &job->dst, np, S_H_OUT0, &d.dst, &e)) return cuda_fail(ctx, e, msg);
     size_t n_luma = (size_t)info.mi_rows * info.mi_cols;
     size_t n_chroma = (size_t)((info.mi_rows + ssy) >> ssy) * ((info.mi_cols + ssx) >> ssx);
     d.tx_luma = stage_array(ctx, S_H_SIDE0, job->tx_luma, n_luma, sc, &e);
@@ -1180,7 +1200,7 @@ static int32_t postfilter_from_host(vaco_av1_ctx* ctx, cudaStream_t s, const vac
         if (job->lr_units[k] && job->lr_unit_count[k] > 0) total_units += (size_t)job->lr_unit_count[k];
     if (e == cudaSuccess && total_units > 0) {
         vaco_av1_lr_unit* du = (vaco_av1_lr_unit*)ctx->scratch(S_H_SIDE5, total_units * sizeof(vaco_av1_lr_unit));
-        if (!du) return cuda_fail(ctx, cudaErrorMemoryAllocation, msg);
+        if (!du) return cudaErrorMemoryAllocation;
         size_t o = 0;
         for (int k = 0; k < 3; ++k) {
             if (job->lr_units[k] && job->lr_unit_count[k] > 0) {
@@ -1192,6 +1212,24 @@ static int32_t postfilter_from_host(vaco_av1_ctx* ctx, cudaStream_t s, const vac
             }
         }
     }
+    return e;
+}
+
+// The chain on a job whose pictures and side information are in host memory:
+// stages the inputs into context scratch, runs the chain into a device
+// picture `*d_out` (context scratch), and leaves the stream synchronized.
+// With sc != s the inputs are copied on stream sc, which `staged` then
+// orders before the chain on s; `defer` is postfilter_dev_impl's.
+static int32_t postfilter_from_host(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_frame_job* job,
+                                    vaco_av1_picture* d_out, int32_t* msg, cudaStream_t sc = nullptr,
+                                    cudaEvent_t staged = nullptr, bool defer = false) {
+    if (!sc) sc = s;
+    const int np = job->info.monochrome ? 1 : 3;
+    cudaError_t e = cudaSuccess;
+    vaco_av1_frame_job d = *job;
+    if (!stage_picture_in(ctx, &job->src, np, S_H_IN0, &d.src, sc, &e)) return cuda_fail(ctx, e, msg);
+    if (!alloc_picture(ctx, &job->dst, np, S_H_OUT0, &d.dst, &e)) return cuda_fail(ctx, e, msg);
+    e = stage_side(ctx, job, d, sc);
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
     if (sc != s) {
         e = cudaEventRecord(staged, sc);
@@ -1203,11 +1241,201 @@ static int32_t postfilter_from_host(vaco_av1_ctx* ctx, cudaStream_t s, const vac
     return st;
 }
 
+// A host job's side information packed into one pinned buffer, so that it goes
+// to the device in one copy: seven small ones take 38 us, one 9.
+struct PackedSide {
+    struct Part {
+        const void* src;
+        size_t at, bytes;
+    };
+    Part parts[8];
+    int n = 0;
+    size_t total = 0;
+
+    // Plans the copy and points the device job `d` at `base` (null: sizes only).
+    void plan(const vaco_av1_frame_job* job, vaco_av1_frame_job* d, unsigned char* base) {
+        const vaco_av1_frame_info& info = job->info;
+        const int np = info.monochrome ? 1 : 3, ssx = info.subsampling_x, ssy = info.subsampling_y;
+        const size_t cells = (size_t)info.mi_rows * info.mi_cols;
+        n = 0;
+        total = 0;
+        auto add = [&](const void* src, size_t bytes) -> unsigned char* {
+            if (!src || bytes == 0) return nullptr;
+            parts[n++] = Part{src, total, bytes};
+            unsigned char* const at = base ? base + total : nullptr;
+            total = align_up(total + bytes, 256);
+            return at;
+        };
+        d->tx_luma = add(job->tx_luma, cells);
+        d->tx_chroma =
+            np > 1 ? add(job->tx_chroma, (size_t)((info.mi_rows + ssy) >> ssy) * ((info.mi_cols + ssx) >> ssx)) : nullptr;
+        d->lvl_map = add(job->lvl_map, cells * 4);
+        d->skip = add(job->skip, cells);
+        d->cdef_idx = reinterpret_cast<const int32_t*>(
+            add(job->cdef_idx, sizeof(int32_t) * (size_t)(job->cdef_count > 0 ? job->cdef_count : 0)));
+        for (int k = 0; k < 3; ++k)
+            d->lr_units[k] = reinterpret_cast<const vaco_av1_lr_unit*>(
+                add(job->lr_units[k], sizeof(vaco_av1_lr_unit) * (size_t)(job->lr_unit_count[k] > 0 ? job->lr_unit_count[k] : 0)));
+    }
+    void pack(unsigned char* host) const {
+        for (int i = 0; i < n; ++i) memcpy(host + parts[i].at, parts[i].src, parts[i].bytes);
+    }
+};
+
+// Bands of tile rows a host frame is filtered in: 1 for a frame with superres
+// (whose picture is upscaled as a whole) and while stages are timed, else one
+// more per kBandBytes of input.  Every band adds its copies' and waits' latency,
+// some 30 us in all, to what it lets overlap.  Calls with 1, 2, 3, 4, 5, 6
+// bands, page-locked buffers: 1080p 10-bit 345, 305, 298, 307, 312, 333 us, 4K
+// 10-bit 1142, 998, 919, 902, 902, 918 us.
+static int host_bands(const vaco_av1_ctx* ctx, const vaco_av1_frame_job* job) {
+    constexpr size_t kBandBytes = 5u << 19;
+    if (job->info.upscaled_width != job->info.coded_width || ctx->timing) return 1;
+    size_t bytes = 0;
+    for (int k = 0; k < (job->info.monochrome ? 1 : 3); ++k) bytes += 2 * (size_t)job->src.width[k] * job->src.height[k];
+    const int tile_rows = div_up(job->info.mi_rows, 16);
+    return (int)std::min<size_t>({bytes / kBandBytes + 1, (size_t)vaco_av1_ctx::kMaxBands, (size_t)tile_rows});
+}
+
+// vaco_av1_postfilter_frame_host, `bands` bands: a band's input rows are copied
+// in while the one before is filtered and the outputs of earlier ones are
+// copied out, on a stream each.  Tile row t needs the input of row t + 1's
+// first samples, so the filters run one tile row behind the copies; a
+// restoration tile needs three rows of CDEF output below it, so it runs with
+// the tile row that holds them.
+static cudaError_t run_bands(vaco_av1_ctx* ctx, const vaco_av1_frame_job* job, int bands,
+                             unsigned long long* host_key) {
+    const vaco_av1_frame_info& info = job->info;
+    const int np = info.monochrome ? 1 : 3, ssy = info.subsampling_y;
+    cudaStream_t s = ctx->stream;
+    cudaError_t e = cudaSuccess;
+    if (!ctx->copy_in) e = cudaStreamCreateWithFlags(&ctx->copy_in, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !ctx->copy_out) e = cudaStreamCreateWithFlags(&ctx->copy_out, cudaStreamNonBlocking);
+    for (int b = 0; b < bands && e == cudaSuccess; ++b) {
+        if (!ctx->band_staged[b]) e = cudaEventCreateWithFlags(&ctx->band_staged[b], cudaEventDisableTiming);
+        if (e == cudaSuccess && !ctx->band_filtered[b])
+            e = cudaEventCreateWithFlags(&ctx->band_filtered[b], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) return e;
+    vaco_av1_frame_job d = *job;
+    if (!alloc_picture(ctx, &job->src, np, S_H_IN0, &d.src, &e)) return e;
+    if (!alloc_picture(ctx, &job->dst, np, S_H_OUT0, &d.dst, &e)) return e;
+    PackedSide side;
+    side.plan(job, &d, nullptr);
+    unsigned char* const side_dev = static_cast<unsigned char*>(ctx->scratch(S_H_SIDE0, std::max<size_t>(side.total, 1)));
+    if (!side_dev) return cudaErrorMemoryAllocation;
+    side.plan(job, &d, side_dev);
+    if (ctx->side_host_bytes < side.total) {
+        if (ctx->side_host) cudaFreeHost(ctx->side_host);
+        ctx->side_host = nullptr;
+        ctx->side_host_bytes = 0;
+        void* p = nullptr;
+        e = cudaMallocHost(&p, side.total);
+        if (e != cudaSuccess) return e;
+        ctx->side_host = static_cast<unsigned char*>(p);
+        ctx->side_host_bytes = side.total;
+    }
+    ChainKernels K;
+    if (postfilter_dev_impl(ctx, s, &d, nullptr, false, &K) != VACO_AV1_OK)
+        return static_cast<cudaError_t>(ctx->last_cuda_error);
+    *host_key = K.host_key;
+
+    // rows [y0, y1) of plane k, host to device or back
+    auto copy_rows = [&](const vaco_av1_picture& dst, const vaco_av1_picture& src, int k, int y0, int y1,
+                         cudaMemcpyKind kind, cudaStream_t on) {
+        if (y0 >= y1 || dst.width[k] <= 0) return cudaSuccess;
+        return cudaMemcpy2DAsync(dst.planes[k] + (size_t)y0 * dst.stride[k], (size_t)dst.stride[k] * 2,
+                                 src.planes[k] + (size_t)y0 * src.stride[k], (size_t)src.stride[k] * 2,
+                                 (size_t)dst.width[k] * 2, (size_t)(y1 - y0), kind, on);
+    };
+    const int tile_rows = div_up(info.mi_rows, 16);
+    int filtered = 0;              // tile rows the fused kernel has run
+    int lr_done[3] = {0, 0, 0};    // tile rows of K.lr[k]
+    int out_rows[vaco_av1_ctx::kMaxBands + 1][3] = {};  // output rows of each plane after band b - 1
+    int t0 = 0;
+    for (int b = 0; b < bands && e == cudaSuccess; ++b) {
+        const bool last = b + 1 == bands;
+        // Bands get smaller: what is left of (1 - x)^2 tile rows, as the last
+        // one's filtering and copy out have nothing to hide behind.
+        const int rest = (bands - 1 - b) * (bands - 1 - b);
+        const int t1 = std::min(std::max(t0 + 1, tile_rows - tile_rows * rest / (bands * bands)),
+                                tile_rows - (bands - 1 - b));
+        for (int k = 0; k < np && e == cudaSuccess; ++k) {
+            const int sy = k ? ssy : 0, h = job->src.height[k];
+            e = copy_rows(d.src, job->src, k, std::min(t0 * (64 >> sy), h), last ? h : std::min(t1 * (64 >> sy), h),
+                          cudaMemcpyHostToDevice, ctx->copy_in);
+        }
+        if (b == 0 && e == cudaSuccess && side.total > 0) {  // packed while the first rows are copied
+            side.pack(ctx->side_host);
+            e = cudaMemcpyAsync(side_dev, ctx->side_host, side.total, cudaMemcpyHostToDevice, ctx->copy_in);
+        }
+        t0 = t1;
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->band_staged[b], ctx->copy_in);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ctx->band_staged[b], 0);
+        const int to = last ? tile_rows : t1 - 1;
+        if (e == cudaSuccess && K.run_db && to > filtered) {
+            K.db.tile_row0 = filtered;
+            K.db.tile_rows = to - filtered;
+            e = launch_dbcdef(K.db, s);
+            ctx->launches++;
+        }
+        filtered = std::max(filtered, to);
+        LrPlane ready[3];
+        int n = 0;
+        for (int i = 0; i < K.nlr; ++i) {
+            LrPlane& p = K.lr[i];
+            const int rows = filtered * (64 >> p.sub_y), all = lr_tile_rows(p);
+            int upto = all;
+            if (!last) upto = std::min(all, std::max(lr_done[i], (rows - 3 + lr_row_offset(p)) / lr_tile_height(p)));
+            if (upto > lr_done[i]) {
+                p.tile_row0 = lr_done[i];
+                p.tile_rows = upto - lr_done[i];
+                ready[n++] = p;
+                lr_done[i] = upto;
+            }
+            out_rows[b + 1][p.plane_index] = last ? p.height : std::max(0, upto * lr_tile_height(p) - lr_row_offset(p));
+        }
+        for (int k = 0; k < np; ++k)
+            if (K.direct[k].out.data)
+                out_rows[b + 1][k] = std::min(filtered * (64 >> (k ? ssy : 0)), K.direct[k].out.height);
+        if (e == cudaSuccess && n > 0) {
+            e = launch_restoration(ready, n, info.bit_depth, ctx->sm_count, s);
+            ctx->launches++;
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->band_filtered[b], s);
+    }
+    // After every input copy is on its way: a copy to pageable memory holds the
+    // calling thread up until it is done.
+    for (int b = 0; b < bands && e == cudaSuccess && K.host_key == kNoError; ++b) {
+        e = cudaStreamWaitEvent(ctx->copy_out, ctx->band_filtered[b], 0);
+        for (int k = 0; k < np && e == cudaSuccess; ++k)
+            e = copy_rows(job->dst, d.dst, k, std::min(out_rows[b][k], job->dst.height[k]),
+                          std::min(out_rows[b + 1][k], job->dst.height[k]), cudaMemcpyDeviceToHost, ctx->copy_out);
+    }
+    return e;
+}
+
 int32_t vaco_av1_postfilter_frame_host(vaco_av1_ctx* ctx, const vaco_av1_frame_job* job, int32_t* msg) {
     if (!ctx || !job) return invalid(msg, VACO_AV1_MSG_NULL_ARGUMENT);
     if (!chain_geometry_ok(job)) return invalid(msg, VACO_AV1_MSG_FRAME_GEOMETRY);
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
+    const int bands = host_bands(ctx, job);
+    if (bands > 1) {
+        unsigned long long host_key = kNoError;
+        cudaError_t e = run_bands(ctx, job, bands, &host_key);
+        // the caller's buffers are its own again once both copy streams are idle
+        for (cudaStream_t c : {ctx->copy_in, ctx->copy_out})
+            if (c) {
+                const cudaError_t w = cudaStreamSynchronize(c);
+                if (e == cudaSuccess) e = w;
+            }
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(s);
+            return cuda_fail(ctx, e, msg);
+        }
+        return finish(ctx, s, host_key, msg);
+    }
     vaco_av1_picture dst;
     const int32_t st = postfilter_from_host(ctx, s, job, &dst, msg);
     if (st != VACO_AV1_OK) return st;

@@ -89,6 +89,13 @@ struct vaco_av1_ctx {
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     uint64_t next_ticket = 1;
 
+    // vaco_av1_postfilter_frame_host in bands of tile rows: a band's input is
+    // on the device / its output rows are written
+    static constexpr int kMaxBands = 5;
+    cudaEvent_t band_staged[kMaxBands] = {}, band_filtered[kMaxBands] = {};
+    unsigned char* side_host = nullptr;  // pinned: a frame's side information, packed
+    size_t side_host_bytes = 0;
+
     // film grain (grain.cu): workspace sets whose template kernels run on
     // their own streams, so the templates of consecutive frames (which depend
     // only on the parameters) overlap each other and the frames' other work

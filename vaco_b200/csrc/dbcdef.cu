@@ -116,6 +116,7 @@ struct DbCdefArgs {
     int staged_vectors;         // 16-byte vectors of all staged planes together
     DirectPlane direct[3];      // final output written here too (see DirectPlane)
     size_t plane_off[3];        // shared-memory offset (samples) of each staged plane
+    int tile_row0;              // first row of tiles of a per-frame launch
 };
 
 // The taps of one lane as words of the staged plane: a pair that starts on an
@@ -732,7 +733,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
 template <int NT, int MIN_CTAS, int LAYOUT, class Block, bool DIRECT = false>
 __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_kernel(DbCdefArgs a) {
     overlap_prologue();
-    dbcdef_tile<NT, LAYOUT, Block, DIRECT>(a, blockIdx.x, blockIdx.y);
+    dbcdef_tile<NT, LAYOUT, Block, DIRECT>(a, blockIdx.x, a.tile_row0 + blockIdx.y);
 }
 
 // Batched form: one CTA per tile of all frames of a batch, frames laid end to
@@ -810,6 +811,7 @@ size_t build_dbcdef_args(const DbCdefLaunch& L, void* out) {
     a.status = L.status;
     a.vec_ok = vec;
     a.dst_vec = dst_vec;
+    a.tile_row0 = L.tile_row0;
     a.staged_vectors = (int)(off / 8);  // each staged plane is a multiple of 8 samples
     for (int p = 0; p < 3; ++p) a.direct[p] = p < np ? L.direct[p] : DirectPlane{};
     memcpy(out, &a, sizeof a);
@@ -883,7 +885,9 @@ cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream) {
     const size_t smem = build_dbcdef_args(L, &a);
     cudaError_t e = dbcdef_kernel_attributes();
     if (e != cudaSuccess) return e;
-    const dim3 grid(div_up(L.info.mi_cols, 16), div_up(L.info.mi_rows, 16));
+    const int tile_rows = L.tile_rows < 0 ? div_up(L.info.mi_rows, 16) - L.tile_row0 : L.tile_rows;
+    if (tile_rows <= 0) return cudaSuccess;
+    const dim3 grid(div_up(L.info.mi_cols, 16), tile_rows);
     const bool direct = a.direct[0].out.data || a.direct[1].out.data || a.direct[2].out.data;
     return a.bit_depth <= 10 ? launch_dbcdef_as<HalfBlock>(a, direct, L.threads, L.sm_count, grid, smem, stream)
                              : launch_dbcdef_as<PairBlock>(a, direct, L.threads, L.sm_count, grid, smem, stream);

@@ -79,7 +79,13 @@ struct LrPlane {
     int copy_only;                  // 1: output = `after` (frame-level restoration off for the plane)
     int plane_index;                // 0 = Y, 1 = U, 2 = V (status-word key of unit checks)
     DeviceStatus* unit_status;      // non-null: validate each tile's unit here (restoration.rs:67-91)
+    int tile_row0 = 0, tile_rows = -1;  // the tile rows to run; -1: all
 };
+// Rows of a plane's tiles and their offset: tile row t covers the plane rows
+// [t * lr_tile_height() - lr_row_offset(), (t + 1) * ...).
+inline int lr_tile_height(const LrPlane& p) { return p.unit_size < (64 >> p.sub_y) ? p.unit_size : 64 >> p.sub_y; }
+inline int lr_row_offset(const LrPlane& p) { return 8 >> p.sub_y; }
+inline int lr_tile_rows(const LrPlane& p) { return div_up(p.height + lr_row_offset(p), lr_tile_height(p)); }
 // A plane whose restoration is off: its tiles only copy `after` into `out`.
 LrPlane copy_only_plane(const DevPlaneC& after, const DevPlane& out, int w, int h, int sub_y, int plane_index);
 // Restores up to 3 planes in one launch.  Units must have been validated.
@@ -156,6 +162,7 @@ struct DbCdefLaunch {
     DeviceStatus* status;
     int threads = 256;          // threads per tile: 256 (512 for frames of few tiles) or 128
     int sm_count = 0;
+    int tile_row0 = 0, tile_rows = -1;  // the rows of 64x64 tiles to run; -1: all
     DirectPlane direct[3] = {};  // per plane; all off unless set
 };
 cudaError_t launch_dbcdef(const DbCdefLaunch& L, cudaStream_t stream);

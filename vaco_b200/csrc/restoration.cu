@@ -87,7 +87,7 @@ struct LrArgs {
     int count;
     int bit_depth;
     const DeviceStatus* guard;  // null, or a status word: an error in it stops every tile
-    int tile_w[3], tile_h[3], tiles_x[3], tiles_y[3], off[3], stripe_h[3];
+    int tile_w[3], tile_h[3], tiles_x[3], tile_y0[3], off[3], stripe_h[3];
     unsigned tiles_x_recip[3], unit_recip[3], stripe_recip[3];  // fast_div_recip of each
     int tile_base[4];
 };
@@ -277,7 +277,9 @@ __device__ __forceinline__ void lr_tile(const LrArgs& a, int block) {
     while (pl + 1 < a.count && block >= a.tile_base[pl + 1]) ++pl;
     const LrPlane& P = a.p[pl];
     const int local = block - a.tile_base[pl];
-    const int ty = (int)fast_div(local, a.tiles_x[pl], a.tiles_x_recip[pl]), tx = local - ty * a.tiles_x[pl];
+    int ty = (int)fast_div(local, a.tiles_x[pl], a.tiles_x_recip[pl]);
+    const int tx = local - ty * a.tiles_x[pl];
+    ty += a.tile_y0[pl];
     const int off = a.off[pl], sh = a.stripe_h[pl];
     const int y_lo = max(ty * a.tile_h[pl] - off, 0);
     const int y_hi = min((ty + 1) * a.tile_h[pl] - off, P.height);
@@ -673,15 +675,16 @@ int build_lr_args(const LrPlane* planes, int count, int bit_depth, void* out) {
         const int sh = 64 >> planes[k].sub_y, off = 8 >> planes[k].sub_y;
         a.stripe_h[k] = sh;
         a.off[k] = off;
-        a.tile_h[k] = min(planes[k].unit_size, sh);
+        a.tile_h[k] = lr_tile_height(planes[k]);
         a.tile_w[k] = min(planes[k].unit_size, kMaxTile);
-        a.tiles_y[k] = div_up(planes[k].height + off, a.tile_h[k]);
+        a.tile_y0[k] = planes[k].tile_row0;
+        const int rows = planes[k].tile_rows < 0 ? lr_tile_rows(planes[k]) - planes[k].tile_row0 : planes[k].tile_rows;
         a.tiles_x[k] = div_up(planes[k].width, a.tile_w[k]);
         a.tiles_x_recip[k] = fast_div_recip((unsigned)a.tiles_x[k]);
         a.unit_recip[k] = fast_div_recip((unsigned)planes[k].unit_size);
         a.stripe_recip[k] = fast_div_recip((unsigned)sh);
         a.tile_base[k] = total;
-        total += a.tiles_x[k] * a.tiles_y[k];
+        total += a.tiles_x[k] * rows;
     }
     for (int k = count; k < 4; ++k) a.tile_base[k] = total;
     memcpy(out, &a, sizeof a);
