@@ -35,36 +35,52 @@ __device__ __forceinline__ uint32_t pack_bytes(uint32_t w) {
     return (lo > 255u ? 0u : lo) | ((hi > 255u ? 0u : hi) << 8);
 }
 
+// A stream: a 4K 10-bit frame reads 24.9 MB and writes as much.  A thread takes
+// kEmitAhead chunks a grid apart and loads all of them before it stores the
+// first, and launches overlap, so the next frame's CTAs start as the last ones
+// of this frame drain.
+constexpr int kEmitAhead = 3;
 __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitArgs a) {
-    const long long total = a.chunk_base[a.count];
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        int p = 0;
-        while (p + 1 < a.count && i >= a.chunk_base[p + 1]) ++p;
-        const EmitPlane& P = a.p[p];
-        const unsigned j = (unsigned)(i - a.chunk_base[p]);  // < 2^31 (checked on the host)
-        const int cpr = a.chunks_per_row[p];
-        const int y = (int)fast_div(j, cpr, a.cpr_recip[p]), x = (int)(j - (unsigned)y * cpr) * 8;
-        const uint16_t* s = P.src + (long)y * P.src_stride + x;
-        uint8_t* d = P.dst + (long long)y * P.dst_stride;
-        const int n = min(8, P.width - x);
-        if (a.vec && n == 8) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(s));
-            if (a.two_bytes) {
-                *reinterpret_cast<uint4*>(d + 2 * x) = q;
+    overlap_prologue();
+    const long long total = a.chunk_base[a.count], step = (long long)gridDim.x * blockDim.x;
+    for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += kEmitAhead * step) {
+        uint4 q[kEmitAhead];
+        uint8_t* d[kEmitAhead];
+        const uint16_t* s[kEmitAhead];
+        int n[kEmitAhead];  // samples of the chunk; 0: none
+#pragma unroll
+        for (int k = 0; k < kEmitAhead; ++k) {
+            const long long i = i0 + k * step;
+            n[k] = 0;
+            if (i >= total) continue;
+            int p = 0;
+            while (p + 1 < a.count && i >= a.chunk_base[p + 1]) ++p;
+            const EmitPlane& P = a.p[p];
+            const unsigned j = (unsigned)(i - a.chunk_base[p]);  // < 2^31 (checked on the host)
+            const int cpr = a.chunks_per_row[p];
+            const int y = (int)fast_div(j, cpr, a.cpr_recip[p]), x = (int)(j - (unsigned)y * cpr) * 8;
+            s[k] = P.src + (long)y * P.src_stride + x;
+            d[k] = P.dst + (long long)y * P.dst_stride + (a.two_bytes ? 2 * x : x);
+            n[k] = min(8, P.width - x);
+            if (a.vec && n[k] == 8) q[k] = __ldg(reinterpret_cast<const uint4*>(s[k]));
+        }
+#pragma unroll
+        for (int k = 0; k < kEmitAhead; ++k) {
+            if (a.vec && n[k] == 8) {
+                if (a.two_bytes)
+                    *reinterpret_cast<uint4*>(d[k]) = q[k];
+                else
+                    *reinterpret_cast<uint2*>(d[k]) = make_uint2(pack_bytes(q[k].x) | (pack_bytes(q[k].y) << 16),
+                                                                 pack_bytes(q[k].z) | (pack_bytes(q[k].w) << 16));
             } else {
-                const uint2 b = make_uint2(pack_bytes(q.x) | (pack_bytes(q.y) << 16),
-                                           pack_bytes(q.z) | (pack_bytes(q.w) << 16));
-                *reinterpret_cast<uint2*>(d + x) = b;
-            }
-        } else {
-            for (int k = 0; k < n; ++k) {
-                const int v = s[k];
-                if (a.two_bytes) {
-                    d[2 * (x + k)] = (uint8_t)(v & 0xFF);
-                    d[2 * (x + k) + 1] = (uint8_t)(v >> 8);
-                } else {
-                    d[x + k] = v > 255 ? 0 : (uint8_t)v;
+                for (int j = 0; j < n[k]; ++j) {
+                    const int v = s[k][j];
+                    if (a.two_bytes) {
+                        d[k][2 * j] = (uint8_t)(v & 0xFF);
+                        d[k][2 * j + 1] = (uint8_t)(v >> 8);
+                    } else {
+                        d[k][j] = v > 255 ? 0 : (uint8_t)v;
+                    }
                 }
             }
         }
@@ -97,8 +113,7 @@ cudaError_t launch_emit(const EmitPlane* planes, int count, int two_bytes, int s
     // with a grid stride.
     const long long want = (total + kEmitThreads - 1) / kEmitThreads;
     const int grid = (int)(want < (long long)sm_count * 8 ? want : (long long)sm_count * 8);
-    emit_kernel<<<grid, kEmitThreads, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_overlapped(emit_kernel, dim3(grid), dim3(kEmitThreads), 0, stream, a);
 }
 
 }  // namespace vaco
