@@ -10,9 +10,9 @@
 //       filtering, and the scaling function of every sample value, written to
 //       a small workspace.
 //       - The templates' random indices come from the spec's 16-bit LFSR.
-//         Each thread takes 16 consecutive samples and starts from the
-//         register value 16 c steps in, which it computes from the seed by
-//         GF(2) matrix products with M^(16 * 2^b) (M = one LFSR step; the
+//         Each thread takes 32 consecutive samples and starts from the
+//         register value 32 c steps in, which it computes from the seed by
+//         GF(2) matrix products with M^(32 * 2^b) (M = one LFSR step; the
 //         host builds those nine matrices), so the sequence needs no
 //         serial walk.
 //       - The AR filter is a wavefront over blocks of four columns; see
