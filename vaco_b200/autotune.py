@@ -50,9 +50,9 @@ def load_tuning() -> dict:
 
 
 # (threads per tile, resident CTAs per SM its body is compiled for) of the
-# fused kernel: the three bodies there are (256 threads at 80 or 64 registers,
-# 128 threads at 5 per SM)
-DBCDEF_SHAPES = ((256, 3), (256, 4), (128, 5))
+# fused kernel's two bodies; the threads choose the body, the second field has
+# no effect
+DBCDEF_SHAPES = ((256, 4), (128, 5))
 
 
 def _time(fn, reps, stream):
