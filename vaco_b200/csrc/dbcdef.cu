@@ -503,8 +503,10 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
                 bad |= t > 18;
                 if (a.lvl_map) {
                     const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(a.lvl_map) + cell);
-                    s_side.lvl[i] = v;
-                    bad |= (v & 0xC0C0C0C0u) != 0;  // a level above 63
+                    // A level above 63 is reported and cut: list entries
+                    // hold 6 bits of it beside the segment's offset.
+                    s_side.lvl[i] = v & 0x3F3F3F3Fu;
+                    bad |= (v & 0xC0C0C0C0u) != 0;
                 }
             }
             if (a.num_planes > 1 && cr0 + wr >= 0 && cc0 + wc >= 0 && cr0 + wr < crows && cc0 + wc < ccols) {
