@@ -70,8 +70,11 @@ int32_t set_msg(int32_t* msg, int m) {
     return m;
 }
 
+// The call's own status reports the error, so it does not stay pending in the
+// thread, where the next launch check or the caller's would take it for its own.
 int32_t cuda_fail(vaco_av1_ctx* ctx, cudaError_t e, int32_t* msg) {
     if (ctx) ctx->last_cuda_error = (int)e;
+    cudaGetLastError();
     set_msg(msg, VACO_AV1_MSG_CUDA);
     return VACO_AV1_DEVICE_ERROR;
 }

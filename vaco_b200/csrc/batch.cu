@@ -95,6 +95,7 @@ DevPlaneC dev_cplane(unsigned char* base, const PlaneBuf& b) {
 
 int32_t fail(vaco_av1_ctx* ctx, cudaError_t e, int32_t* statuses, int32_t* msgs, int n) {
     ctx->last_cuda_error = (int)e;
+    cudaGetLastError();  // reported by the call: not pending for the next one
     for (int i = 0; i < n; ++i) {
         if (statuses) statuses[i] = VACO_AV1_DEVICE_ERROR;
         if (msgs) msgs[i] = VACO_AV1_MSG_CUDA;
