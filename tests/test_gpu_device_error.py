@@ -59,3 +59,24 @@ def test_device_error_is_reported_once(own_ctx, batch, oracle_threads):
                                               C.byref(msg)) == abi.OK
     torch.cuda.synchronize()
     same([t.cpu().numpy().view(np.uint16) for t in d.planes], want, "deblock")
+
+
+def test_call_that_failed_half_way_leaves_the_next_one_alone(own_ctx, oracle_threads):
+    """A frame with a bad sample fails while its first kernel is still queued
+    behind other work.  What that kernel reports later is not the next call's error."""
+    import torch
+
+    f = synth.make_small(31, 200, 136, 10)
+    want, m = oracle.postfilter_frame(f, threads=oracle_threads)
+    assert m == 0
+    good = DeviceFrame(f)
+    own_ctx.postfilter_frame_dev(good)  # the scratch both calls share is there
+    f.planes[0][40, 33] = 1 << 10
+    bad = too_wide(f)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # about 0.1 s on the stream of both calls
+    with pytest.raises(VacoError) as e:
+        own_ctx.postfilter_frame_dev(bad)
+    assert e.value.status == abi.DEVICE_ERROR
+    own_ctx.postfilter_frame_dev(good)
+    same(good.outputs_numpy(), want, "next frame")

@@ -85,18 +85,16 @@ int32_t invalid(int32_t* msg, int m) {
                                                                                 : VACO_AV1_INVALID_DATA;
 }
 
-// Starts a call from a clean status word.  The word is clean unless its flag
-// is up (a call that failed half-way left its kernels' report unread), or the
-// context defers status: then it may hold earlier frames' errors, which a call
-// that returns its own status drops.
+// Starts a call from a clean status word.  The word is clean when the call
+// before was waited for and its report, if any, taken by finish().  It may not
+// be after a call that failed half-way, whose kernels can still be running and
+// report later, and while the context defers status, where it may hold earlier
+// frames' errors, which a call that returns its own status drops: then it is
+// reset in stream order.
 cudaError_t reset_status(vaco_av1_ctx* ctx, cudaStream_t s) {
-    if (!ctx->deferred && *ctx->status_flag == 0) return cudaSuccess;
-    if (!ctx->deferred) {
-        const cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return e;
-        *ctx->status_flag = 0;
-    }
-    return cudaMemsetAsync(ctx->status, 0xFF, sizeof(unsigned long long), s);
+    const bool clean = !ctx->deferred && !ctx->status_open && *ctx->status_flag == 0;
+    ctx->status_open = true;
+    return clean ? cudaSuccess : cudaMemsetAsync(ctx->status, 0xFF, sizeof(unsigned long long), s);
 }
 
 // Waits for the stream, reads the status word back when a kernel raised its
@@ -114,6 +112,7 @@ int32_t finish(vaco_av1_ctx* ctx, cudaStream_t s, unsigned long long host_key, i
         if (!ctx->deferred) *ctx->status_flag = 0;
         key = *ctx->status_host;
     }
+    ctx->status_open = false;
     ctx->collect_marks();
     if (host_key < key) key = host_key;
     if (key == kNoError) {
@@ -442,6 +441,7 @@ int32_t vaco_av1_ctx_set_deferred_status(vaco_av1_ctx* ctx, int32_t enable) {
         cudaMemset(ctx->status, 0xFF, sizeof(unsigned long long)) != cudaSuccess)
         return VACO_AV1_DEVICE_ERROR;
     *ctx->status_flag = 0;
+    ctx->status_open = false;
     ctx->deferred = enable != 0;
     return VACO_AV1_OK;
 }
