@@ -86,11 +86,11 @@ int32_t invalid(int32_t* msg, int m) {
 }
 
 // Starts a call from a clean status word.  The word is clean when the call
-// before was waited for and its report, if any, taken by finish().  It may not
-// be after a call that failed half-way, whose kernels can still be running and
-// report later, and while the context defers status, where it may hold earlier
-// frames' errors, which a call that returns its own status drops: then it is
-// reset in stream order.
+// before was waited for and reported nothing.  It holds that call's error
+// otherwise, may still get one from a call that failed half-way, whose kernels
+// can be running, and earlier frames' errors while the context defers status,
+// which a call that returns its own status drops: then it is reset in stream
+// order.
 cudaError_t reset_status(vaco_av1_ctx* ctx, cudaStream_t s) {
     const bool clean = !ctx->deferred && !ctx->status_open && *ctx->status_flag == 0;
     ctx->status_open = true;
@@ -105,14 +105,12 @@ int32_t finish(vaco_av1_ctx* ctx, cudaStream_t s, unsigned long long host_key, i
     unsigned long long key = kNoError;
     if (*ctx->status_flag) {
         e = cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && !ctx->deferred)
-            e = cudaMemsetAsync(ctx->status, 0xFF, sizeof(unsigned long long), s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
         if (!ctx->deferred) *ctx->status_flag = 0;
         key = *ctx->status_host;
     }
-    ctx->status_open = false;
+    ctx->status_open = key != kNoError;
     ctx->collect_marks();
     if (host_key < key) key = host_key;
     if (key == kNoError) {
@@ -450,7 +448,9 @@ int32_t vaco_av1_ctx_flush(vaco_av1_ctx* ctx, void* stream, int32_t* msg) {
     if (!ctx) return invalid(msg, VACO_AV1_MSG_NULL_ARGUMENT);
     cudaSetDevice(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
+    const bool open = ctx->status_open;
     const int32_t st = finish(ctx, s, kNoError, msg);
+    ctx->status_open |= open;  // nothing reset the word here
     if (st == VACO_AV1_DEVICE_ERROR || *ctx->status_flag == 0) return st;
     cudaError_t e = reset_status(ctx, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

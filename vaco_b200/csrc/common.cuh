@@ -34,8 +34,8 @@ enum Stage : unsigned { STAGE_DEBLOCK = 0, STAGE_CDEF = 1, STAGE_SUPERRES = 2, S
 __device__ __forceinline__ void report_error(DeviceStatus* st, unsigned stage,
                                              unsigned long long position, unsigned msg) {
     unsigned long long key = ((unsigned long long)stage << 60) | ((position & ((1ull << 52) - 1)) << 8) | msg;
-    atomicMin(&st->first_error, key);
-    if (st->host_flag) *static_cast<volatile unsigned*>(st->host_flag) = 1u;
+    if (atomicMin(&st->first_error, key) == kNoError && st->host_flag)
+        *static_cast<volatile unsigned*>(st->host_flag) = 1u;
 }
 
 // ---------------------------------------------------------------- overlapped launches

@@ -19,10 +19,10 @@ struct vaco_av1_ctx {
     vaco::DeviceStatus* status = nullptr;     // device
     unsigned long long* status_host = nullptr;  // pinned
     // Raised by the kernels that report into `status` (see DeviceStatus).
-    // While it is down and no call is open the word holds "no error", so
-    // nothing resets it.
+    // While it is down and status_open is false the word holds "no error",
+    // so nothing resets it.
     volatile unsigned* status_flag = nullptr;   // pinned
-    bool status_open = false;                   // a call began to report and has not come to finish()
+    bool status_open = false;                   // the last call reported an error, or was not waited for
     int last_cuda_error = 0;
     uint64_t launches = 0;
     // deferred status (vaco_av1_ctx_set_deferred_status): chain calls on
