@@ -577,10 +577,8 @@ int32_t vaco_av1_cdef_picture_dev(vaco_av1_ctx* ctx, void* stream, const vaco_av
         all_zero = all_zero && params->y_primary[k] == 0 && params->y_secondary[k] == 0 && params->uv_primary[k] == 0 &&
                    params->uv_secondary[k] == 0;
     if (params->enabled && !all_zero && skip && (cdef_idx || cdef_count <= 0) && fused_takes(*src, *dst, *info)) {
-        // The fused kernel with deblocking off.  It checks more than
-        // apply_cdef does (every sample, where vaco looks at the filtered
-        // blocks alone) and names the error less closely, so a picture that
-        // it objects to goes to the per-stage kernel below, whose word counts.
+        // The fused kernel with deblocking off: without transform sizes it
+        // makes apply_cdef's checks alone.  1080p 10-bit 4:2:0 67 -> 36 us a call.
         DbCdefLaunch L{};
         L.src = *src;
         L.dst = *dst;
@@ -592,10 +590,7 @@ int32_t vaco_av1_cdef_picture_dev(vaco_av1_ctx* ctx, void* stream, const vaco_av
         L.cdef = *params;
         e = run_fused(ctx, s, L);
         if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
-        const int32_t st = finish(ctx, s, kNoError, msg);
-        if (st != VACO_AV1_INVALID_DATA) return st;
-        e = reset_status(ctx, s);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, msg);
+        return finish(ctx, s, kNoError, msg);
     }
     unsigned long long hk = run_cdef(ctx, s, *src, *dst, *info, skip, cdef_idx, cdef_stride, cdef_count, *params, &e);
     if (e != cudaSuccess) return cuda_fail(ctx, e, msg);

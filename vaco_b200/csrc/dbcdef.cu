@@ -381,10 +381,38 @@ __device__ __forceinline__ void deblock_filter(const DbCdefArgs& a, int ssx, int
     __syncthreads();
 }
 
+// The samples that vaco checks for a filtered block (decode.rs:780-841): the
+// block's own luma, then, with a valid strength index, every plane's that its
+// taps can reach.  Reports the first above the bit depth; the block's other
+// checks have the same keys where they are made.  (Staged samples past the
+// plane's borders are copies of ones inside the same reach.)
+__device__ __forceinline__ void report_bad_block(const DbCdefArgs& a, int ssx, int ssy, const uint16_t* smem, int b,
+                                                 int index, int mi_r0, int mi_c0) {
+    const int by = b >> 3, bx = b & 7;
+    const unsigned long long pos = ((unsigned long long)(mi_r0 + 2 * by) * a.mi_cols + mi_c0 + 2 * bx) * 4;
+#pragma unroll 1
+    for (int k = 0; k <= (index < 8 ? a.num_planes : 0); ++k) {  // luma alone, then the planes with their reach
+        const PlaneGeom g = plane_geom(k > 1 ? 1 : 0, ssx, ssy);
+        const int bw = 8 >> g.sx, bh = 8 >> g.sy, reach = k ? 2 : 0;
+        const uint16_t* t =
+            smem + a.plane_off[max(k - 1, 0)] + (kHalo + by * bh - reach) * g.pitch + kHalo + bx * bw - reach;
+        int most = 0;
+#pragma unroll 1
+        for (int i = 0; i < (bh + 2 * reach) * (bw + 2 * reach); ++i)
+            most = max(most, (int)t[i / (bw + 2 * reach) * g.pitch + i % (bw + 2 * reach)]);
+        if (most >> a.bit_depth) {
+            report_error(a.status, STAGE_CDEF, pos + k, k ? VACO_AV1_MSG_CDEF_BLOCK_PARAMS : VACO_AV1_MSG_CDEF_SAMPLE);
+            return;
+        }
+    }
+}
+
 // One 64x64 filter block (tile_x, tile_y) of one frame.  Every thread of the
 // CTA calls it; it ends with all threads past their last shared-memory use
 // only after the caller's next __syncthreads().
-template <int NT, int LAYOUT, class Block, bool DIRECT = false>
+// ALONE: the call may be cdef_picture's, for CDEF alone, which has no transform
+// sizes.
+template <int NT, int LAYOUT, class Block, bool DIRECT, bool ALONE>
 __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int tile_y) {
     constexpr int kWarpsNT = NT / 32;
     constexpr bool kHalf = std::is_same<Block, HalfBlock>::value;  // samples of up to 10 bits
@@ -489,7 +517,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     // copies are in flight (cells the two passes touch; see SideWindow).  Each
     // cell is checked where it is loaded: the windows of all tiles together
     // hold exactly the maps' cells.
-    if (a.tx_luma) {  // null for CDEF alone
+    if (!ALONE || a.tx_luma) {
         const int crows = (a.mi_rows + ssy) >> ssy, ccols = (a.mi_cols + ssx) >> ssx;
         const int cr0 = (mi_r0 >> ssy) - kWinTop, cc0 = (mi_c0 >> ssx) - kWinLeft;
         int bad = 0;
@@ -520,12 +548,12 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     const bool any_active = __syncthreads_or(act);
 
+    // ---- input check from shared memory
+    // Every staged sample, halo included: the halo holds samples of the
+    // same planes (edge-clamped copies past their borders), so the tiles
+    // together check exactly the planes' samples, and a flat pass over
+    // the staged vectors needs no per-row indexing.
     {
-        // ---- input check from shared memory
-        // Every staged sample, halo included: the halo holds samples of the
-        // same planes (edge-clamped copies past their borders), so the tiles
-        // together check exactly the planes' samples, and a flat pass over
-        // the staged vectors needs no per-row indexing.
         const uint32_t hi = ((0xFFFFu << a.bit_depth) & 0xFFFFu) * 0x10001u;  // bits above the depth, per lane
         const uint4* v = reinterpret_cast<const uint4*>(smem);
         uint32_t acc = 0;
@@ -535,8 +563,10 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         }
         // A report a warp: one a thread, all to one word, took a 4K frame of
         // bad samples alone from 161 to 431 us.
-        if (__any_sync(0xFFFFFFFFu, (acc & hi) != 0) && lane == 0)
-            report_error(a.status, STAGE_DEBLOCK, 1, VACO_AV1_MSG_DB_SAMPLE);
+        if (__any_sync(0xFFFFFFFFu, (acc & hi) != 0) && lane == 0) {
+            if (ALONE && !a.tx_luma) s_count[0] = 1;  // without deblocking nothing else counts there
+            else report_error(a.status, STAGE_DEBLOCK, 1, VACO_AV1_MSG_DB_SAMPLE);
+        }
     }
 
     // ---- deblocking, pass 0 (vertical edges) then pass 1 (horizontal edges)
@@ -549,6 +579,10 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
         // the sample check above reads every staged sample, the sentinel
         // phase below overwrites some
         __syncthreads();
+        if (ALONE && !a.tx_luma && s_count[0]) {  // a bad sample: apply_cdef's rule
+            if (tid < 64 && s_active[tid]) report_bad_block(a, ssx, ssy, smem, tid, index, mi_r0, mi_c0);
+            __syncthreads();
+        }
     }
 
     // ---- stripe-boundary rows of the deblocked picture for restoration: rows
@@ -738,7 +772,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
 template <int NT, int MIN_CTAS, int LAYOUT, class Block, bool DIRECT = false>
 __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_kernel(DbCdefArgs a) {
     overlap_prologue();
-    dbcdef_tile<NT, LAYOUT, Block, DIRECT>(a, blockIdx.x, a.tile_row0 + blockIdx.y);
+    dbcdef_tile<NT, LAYOUT, Block, DIRECT, !DIRECT>(a, blockIdx.x, a.tile_row0 + blockIdx.y);
 }
 
 // Batched form: one CTA per tile of all frames of a batch, frames laid end to
@@ -756,7 +790,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) dbcdef_batch_kernel(const DbCdef
     const DbCdefArgs& a = frames[f];
     const int local = blockIdx.x - tile_prefix[f];
     const int tiles_x = (a.mi_cols + 15) / 16;
-    dbcdef_tile<NT, LAYOUT, Block>(a, local % tiles_x, local / tiles_x);
+    dbcdef_tile<NT, LAYOUT, Block, false, false>(a, local % tiles_x, local / tiles_x);
 }
 
 }  // namespace
