@@ -1280,22 +1280,38 @@ struct PackedSide {
     }
 };
 
-// Bands of tile rows a host frame is filtered in: 1 for a frame with superres
-// (whose picture is upscaled as a whole) and while stages are timed, else one
-// more per kBandBytes of input.  Every band adds its copies' and waits' latency,
-// some 30 us in all, to what it lets overlap.  Calls with 1, 2, 3, 4, 5, 6
-// bands, page-locked buffers: 1080p 10-bit 345, 305, 298, 307, 312, 333 us, 4K
-// 10-bit 1142, 998, 919, 902, 902, 918 us.
+// Bands of tile rows a host frame is filtered in: 0, the plain sequence of
+// postfilter_from_host(), for a frame with superres (whose picture is upscaled
+// as a whole), while stages are timed and for less than kBandBytes of input,
+// else one more per kBandBytes.  Every band adds its copies' and waits' latency,
+// some 30 us in all, to what it lets overlap.  Calls with 1, 2, 3, 4, 5, 6 bands,
+// page-locked buffers: 1080p 10-bit 345, 305, 298, 307, 312, 333 us, 4K 10-bit
+// 1142, 998, 919, 902, 902, 918 us.
+// Copies of pageable memory hold the calling thread up, so bands overlap little
+// of them and add copies: one band then, which still packs the side information.
+// 1080p 10-bit 894 us in three bands, 788 in one; 4K 10-bit 3070 in five, 2743 in
+// one; with only one side page-locked 692 and 661, 1955 and 1923 (source), 548
+// and 525, 1970 and 1934 (output).
 static int host_bands(const vaco_av1_ctx* ctx, const vaco_av1_frame_job* job) {
     constexpr size_t kBandBytes = 5u << 19;
-    if (job->info.upscaled_width != job->info.coded_width || ctx->timing) return 1;
+    if (job->info.upscaled_width != job->info.coded_width || ctx->timing) return 0;
+    const int np = job->info.monochrome ? 1 : 3;
     size_t bytes = 0;
-    for (int k = 0; k < (job->info.monochrome ? 1 : 3); ++k) bytes += 2 * (size_t)job->src.width[k] * job->src.height[k];
+    for (int k = 0; k < np; ++k) bytes += 2 * (size_t)job->src.width[k] * job->src.height[k];
     const int tile_rows = div_up(job->info.mi_rows, 16);
-    return (int)std::min<size_t>({bytes / kBandBytes + 1, (size_t)vaco_av1_ctx::kMaxBands, (size_t)tile_rows});
+    const int bands =
+        (int)std::min<size_t>({bytes / kBandBytes + 1, (size_t)vaco_av1_ctx::kMaxBands, (size_t)tile_rows});
+    if (bands == 1) return 0;
+    for (int k = 0; k < np; ++k)
+        for (const uint16_t* p : {job->src.planes[k], job->dst.planes[k]}) {
+            cudaPointerAttributes attr{};
+            if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) cudaGetLastError();
+            if (attr.type == cudaMemoryTypeUnregistered) return 1;
+        }
+    return bands;
 }
 
-// vaco_av1_postfilter_frame_host, `bands` bands: a band's input rows are copied
+// vaco_av1_postfilter_frame_host in `bands` bands: a band's input rows are copied
 // in while the one before is filtered and the outputs of earlier ones are
 // copied out, on a stream each.  Tile row t needs the input of row t + 1's
 // first samples, so the filters run one tile row behind the copies; a
@@ -1419,7 +1435,7 @@ int32_t vaco_av1_postfilter_frame_host(vaco_av1_ctx* ctx, const vaco_av1_frame_j
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
     const int bands = host_bands(ctx, job);
-    if (bands > 1) {
+    if (bands > 0) {
         unsigned long long host_key = kNoError;
         cudaError_t e = run_bands(ctx, job, bands, &host_key);
         // the caller's buffers are its own again once both copy streams are idle
