@@ -11,7 +11,7 @@
 // that no tap can use: constrain() of a sentinel difference is 0 and the
 // maximum masks it out, which is exactly vaco's "unavailable border samples
 // are ignored" rule (the availability edges of apply_cdef are the plane
-// bounds, decode.rs:828-831).
+// bounds, decode.rs:828-831; see load_tile() for planes that end inside a block).
 #include "cdef_core.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
@@ -43,18 +43,23 @@ struct CdefFrameArgs {
 };
 
 // Stage tile rows [y0-2, y0+h+2) x cols [x0-8, x0+w+8) of plane p into smem.
-// Returns (via *bad) whether an in-plane sample exceeds the bit depth.
+// Returns (via *bad) whether an in-plane sample exceeds the bit depth.  With an
+// odd count of mode-info cells the plane's last blocks (bw x bh samples) reach
+// past it: what they have there repeats the plane's edge (framebuf.rs:50-59) and
+// counts as available, as apply_cdef's edges are those of the whole blocks.
 __device__ __forceinline__ void load_tile(uint16_t* sm, int pitch, int rows, const DevPlaneC& p, int x0,
-                                          int y0, int limit, bool vec, int* bad) {
+                                          int y0, int bw, int bh, int limit, bool vec, int* bad) {
     const int vecs_per_row = pitch / 8;
+    const int width = (p.width + bw - 1) & -bw, height = (p.height + bh - 1) & -bh;  // of the blocks
     int local_bad = 0;
     for (int v = threadIdx.x; v < rows * vecs_per_row; v += blockDim.x) {
         int r = v / vecs_per_row, cv = v - r * vecs_per_row;
         int y = y0 - 2 + r, x = x0 - 8 + cv * 8;
         uint16_t* d = sm + r * pitch + cv * 8;
-        bool row_in = y >= 0 && y < p.height;
+        bool row_in = y >= 0 && y < height;
+        const uint16_t* row = p.data + (long)min(y, p.height - 1) * p.stride;
         if (vec && row_in && x >= 0 && x + 8 <= p.width) {
-            uint4 q = __ldg(reinterpret_cast<const uint4*>(p.data + (long)y * p.stride + x));
+            uint4 q = __ldg(reinterpret_cast<const uint4*>(row + x));
             *reinterpret_cast<uint4*>(d) = q;
             uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -64,8 +69,8 @@ __device__ __forceinline__ void load_tile(uint16_t* sm, int pitch, int rows, con
             for (int k = 0; k < 8; ++k) {
                 int xx = x + k;
                 int s = kSent;
-                if (row_in && xx >= 0 && xx < p.width) {
-                    s = __ldg(p.data + (long)y * p.stride + xx);
+                if (row_in && xx >= 0 && xx < width) {
+                    s = __ldg(row + min(xx, p.width - 1));
                     local_bad |= s > limit;
                 }
                 d[k] = (uint16_t)s;
@@ -117,9 +122,10 @@ __global__ void __launch_bounds__(kThreads) cdef_frame_kernel(CdefFrameArgs a) {
     const int limit = a.bd_ok ? (1 << a.bit_depth) - 1 : 0xFFFF;
     const bool vec = a.vec_ok != 0;
     if (s_any) {
-        load_tile(tile[0], kLumaPitch, kLumaRows, a.src[0], x0, y0, limit, vec, &s_bad);
+        load_tile(tile[0], kLumaPitch, kLumaRows, a.src[0], x0, y0, 8, 8, limit, vec, &s_bad);
         for (int p = 1; p < a.num_planes; ++p)
-            load_tile(tile[p], cpitch, crows, a.src[p], x0 >> a.ssx, y0 >> a.ssy, limit, vec, &s_bad);
+            load_tile(tile[p], cpitch, crows, a.src[p], x0 >> a.ssx, y0 >> a.ssy, 8 >> a.ssx, 8 >> a.ssy, limit, vec,
+                      &s_bad);
     }
     __syncthreads();
 
