@@ -60,3 +60,17 @@ def test_deblock(ctx, cut, bd, layout, oracle_threads):
     want, m = oracle.deblock_picture(f, threads=oracle_threads)
     assert m == 0
     same(ctx.deblock_picture(f), want)
+
+
+@pytest.mark.parametrize("layout", LAYOUTS, ids=["420", "422", "444", "mono"])
+@pytest.mark.parametrize("cut", [(1, 0), (0, 1), (1, 1)], ids=["rows", "cols", "both"])
+def test_deblock_with_a_level_map(ctx, cut, layout, oracle_threads):
+    """A subsampled chroma cell's levels are those of its last luma cell, which
+    the map's last cells have not: its last row and column stand in.  The map
+    holds the frame's levels throughout, so the result is the one without it."""
+    f = cell_frame(6, 200, 136, 10, cut, subsampling=layout[:2], monochrome=layout[2])
+    f.deblock_levels = (30, 24, 41, 17)
+    want, m = oracle.deblock_picture(f, threads=oracle_threads)
+    assert m == 0
+    f.lvl_map = np.tile(np.array(f.deblock_levels, np.uint8), (*f.cells, 1))
+    same(ctx.deblock_picture(f), want)

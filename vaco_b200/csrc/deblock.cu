@@ -50,7 +50,7 @@ __global__ void deblock_vertical_kernel(PassArgs a) {
     if (xp & ((1 << wl) - 1)) return;
     const int base = min(wl, tx_w_log2(prev));
     const int size = min(plane ? 8 : 16, 1 << base);
-    const int r = row | ssy, c = col | ssx;
+    const int r = min(row | ssy, L.mi_rows - 1), c = min(col | ssx, L.mi_cols - 1);  // odd counts end early
     int lvl = level_at(L, plane, 0, r, c);
     if (lvl == 0) lvl = level_at(L, plane, 0, r, c - (1 << ssx));
     if (lvl == 0) return;
@@ -77,7 +77,7 @@ __global__ void deblock_horizontal_kernel(PassArgs a) {
     if (yp & ((1 << hl) - 1)) return;
     const int base = min(hl, tx_h_log2(prev));
     const int size = min(plane ? 8 : 16, 1 << base);
-    const int r = row | ssy, c = col | ssx;
+    const int r = min(row | ssy, L.mi_rows - 1), c = min(col | ssx, L.mi_cols - 1);  // odd counts end early
     int lvl = level_at(L, plane, 1, r, c);
     if (lvl == 0) lvl = level_at(L, plane, 1, r - (1 << ssy), c);
     if (lvl == 0) return;
