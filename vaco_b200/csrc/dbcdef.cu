@@ -49,7 +49,6 @@ constexpr int kListTotal = 2380;
 // Rows of the luma CDEF window (th + 4) kept as odd-aligned pairs, and the
 // words of luma's and both 4:2:0 chroma planes' (see shift_copy()).
 constexpr int kShiftRows = 64 + 4;
-constexpr bool kShiftChroma = true;
 constexpr int kShiftWords = kShiftRows * (64 + 2 * kHalo) / 2 + 2 * (32 + 2 * kHalo) * (32 + 2 * kHalo) / 2;
 
 // Side-information window of a tile: cells [mi_r0 - kWinTop, +kWinRows) x
@@ -668,7 +667,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     // aligned load: luma, and 4:2:0 chroma, whose copies lie as far apart as
     // the staged planes (the other layouts' do not fit beside luma's).
     shift_copy<64 + 2 * kHalo, kShiftRows, NT>(smem + a.plane_off[0], s_u.shifted);
-    if (kShiftChroma && a.num_planes > 1 && ssx == 1 && ssy == 1) {
+    if (a.num_planes > 1 && ssx == 1 && ssy == 1) {
         uint32_t* sc = s_u.shifted + kShiftRows * (64 + 2 * kHalo) / 2;
         shift_copy<32 + 2 * kHalo, 32 + 4, NT>(smem + a.plane_off[1], sc);
         shift_copy<32 + 2 * kHalo, 32 + 4, NT>(smem + a.plane_off[2], sc + (32 + 2 * kHalo) * (32 + 2 * kHalo) / 2);
@@ -749,7 +748,7 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
                     a, 1, tc, nullptr, plane_words, px0, py0, s_active, s_block[1], c_pri_on, c_sec_on, br, part, lane,
                     ssx);
             else if (ssy == 1)
-                filter_block_row<32 + 2 * kHalo, 4, 2, 2, kParts, kShiftChroma, DIRECT>(
+                filter_block_row<32 + 2 * kHalo, 4, 2, 2, kParts, true, DIRECT>(
                     a, 1, tc, s_u.shifted + kShiftRows * (64 + 2 * kHalo) / 2, plane_words, px0, py0, s_active,
                     s_block[1], c_pri_on, c_sec_on, br, part, lane, ssx);
             else

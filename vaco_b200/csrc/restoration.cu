@@ -115,8 +115,6 @@ constexpr size_t lr_smem(int threads) {
     return kSBytes + kRegion + 256 * sizeof(uint16_t) + sizeof(int32_t) * 2 * kVCols * (threads / 32);
 }
 
-__device__ __forceinline__ int round2i(int v, int s) { return s == 0 ? v : (v + (1 << (s - 1))) >> s; }
-
 __device__ __forceinline__ bool unit_ok(const vaco_av1_lr_unit& u) {
     if (u.type == VACO_AV1_LR_NONE) return true;
     if (u.type == VACO_AV1_LR_WIENER) {
