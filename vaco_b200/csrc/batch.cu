@@ -510,12 +510,15 @@ int32_t vaco::batch_enqueue(vaco_av1_ctx* ctx, cudaStream_t s, const vaco_av1_fr
             launches += 1 + plan[i].np + (jobs[i].deblock.levels[0] || jobs[i].deblock.levels[1] ? 2 : 0) + 1;
     }
     ctx->mark(0, s);
-    const bool graphs = ctx->tuning.use_graphs && s != nullptr;
+    // The per-stage kernels take the frames' pointers and levels by value, which
+    // a replay would not renew: graphs are for the fused kernels, whose tables it
+    // uploads.
+    const bool graphs = ctx->tuning.use_graphs && fused && s != nullptr;
     if (graphs) {
         signature += "@" + std::to_string(ctx->scratch_generation) + "/" +
                      std::to_string(ctx->tuning.dbcdef_ctas_per_sm) + "/" + std::to_string(ctx->tuning.lr_ctas_per_sm) +
                      "/" + std::to_string(ctx->tuning.largest_first) + "/" +
-                     std::to_string(ctx->tuning.dbcdef_threads) + "/" + std::to_string(ctx->tuning.stage_fusion);
+                     std::to_string(ctx->tuning.dbcdef_threads);
         auto it = ctx->graphs.find(signature);
         if (it == ctx->graphs.end()) {
             // kernel attributes are set outside the capture
