@@ -19,8 +19,8 @@
  *     returning.  `*_dev` entry points take device pointers and only enqueue
  *     work on `stream` (a cudaStream_t, NULL = the legacy default stream); the
  *     status they return covers argument checks, launch errors and the data
- *     checks, which need one small device-to-host read of a status word, so a
- *     `*_dev` call synchronizes `stream` once before returning.
+ *     checks, so a `*_dev` call synchronizes `stream` once before returning.
+ *     A status word is read back only when a kernel reported an error.
  *   - Every entry point returns a status (vaco_av1_status) and, when `msg` is
  *     non-NULL, stores a message id (vaco_av1_msg) naming the failed check;
  *     vaco_av1_message() maps it to the same text vaco's
@@ -391,7 +391,10 @@ typedef struct vaco_av1_frame_job {
 /* deblock -> CDEF -> superres (when upscaled_width != coded_width) -> loop
  * restoration for one frame.  The output is the picture vaco's decode_frame
  * would hand to pic_to_frame, cropped to the visible size; subsampled frames
- * need even coded/upscaled widths and heights. */
+ * need even coded/upscaled widths and heights.
+ * _host: large frames whose planes are all in page-locked memory (registered,
+ * or allocated so) are copied and filtered in bands that overlap; frames in
+ * pageable memory are copied whole. */
 VACO_AV1_API int32_t vaco_av1_postfilter_frame_dev(vaco_av1_ctx* ctx, void* stream,
                                       const vaco_av1_frame_job* job, int32_t* msg);
 VACO_AV1_API int32_t vaco_av1_postfilter_frame_host(vaco_av1_ctx* ctx, const vaco_av1_frame_job* job,
@@ -405,13 +408,17 @@ typedef struct vaco_av1_tuning {
     int32_t dbcdef_ctas_per_sm;  /* 1..8; without effect: the batched deblock+CDEF kernel
                                     has one register budget per threads a tile */
     int32_t lr_ctas_per_sm;      /* resident CTAs per SM the batched restoration kernel is
-                                    compiled for, i.e. its register budget (1..8): up to
-                                    3 -> 80 registers a thread, 4 and more -> 64 */
-    int32_t use_graphs;          /* capture each batch composition once as a CUDA graph */
+                                    compiled for (1..8): up to 3 -> a body that takes 66
+                                    registers a thread, so 3 CTAs fit; 4 and more -> 64,
+                                    4 fit (5 % faster on the mix of frames) */
+    int32_t use_graphs;          /* capture each batch composition once as a CUDA graph
+                                    (with stage_fusion) */
     int32_t largest_first;       /* lay the largest frames' tiles first in the launch */
     int32_t dbcdef_threads;      /* threads per 64x64 tile of the deblock+CDEF kernel, in the
                                     batched form and vaco_av1_postfilter_frame_dev: 256 or
-                                    128 (0 = 256) */
+                                    128 (0 = 256; 128 is 13 to 15 % slower).  With 256, a
+                                    frame of up to two tiles per SM takes 512 in a call of
+                                    its own */
     int32_t stage_fusion;        /* batched form: 1 = deblocking and CDEF in one fused
                                     kernel; 0 = as separate per-stage kernels, frame by
                                     frame */
@@ -631,10 +638,11 @@ typedef struct vaco_av1_film_grain_params {
  * VACO_AV1_MSG_FRAME_GEOMETRY for planes smaller than the frame, and with
  * VACO_AV1_MSG_FG_SAMPLE when a sample of `in` exceeds the bit depth.
  * apply_grain == 0 copies `in` to `out`.  `in` and `out` may not overlap.
- * The grain templates depend only on `params`; they are built on one of the
- * context's internal streams (one per workspace set, eight sets used in
- * turn), ordered against `stream` by events, so consecutive frames' template
- * builds overlap each other and the frames' other work.
+ * The grain templates depend only on `params`.  With deferred status they are
+ * built on one of the context's internal streams (one per workspace set, eight
+ * sets used in turn), ordered against `stream` by events, so consecutive
+ * frames' template builds overlap each other and the frames' other work; a call
+ * that waits for its frame runs both of its kernels on `stream`.
  * _dev: device pointers, runs on `stream` and synchronizes it for the
  * status, unless the context has deferred status enabled (then it only
  * enqueues; vaco_av1_ctx_flush reports).  _host: host pointers,

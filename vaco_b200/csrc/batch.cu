@@ -12,7 +12,7 @@
 //      also validates every restoration unit and copies planes whose
 //      frame-level restoration is off
 //   5. the per-frame status words, read only when a kernel raised the batch flag
-// With tuning.use_graphs, steps 1-5 are captured once per batch composition as
+// With tuning.use_graphs, steps 1-4 are captured once per batch composition as
 // a CUDA graph and replayed afterwards; the tables carry every per-batch
 // pointer, so a replay only needs the host to refresh the pinned staging copy.
 #include <algorithm>

@@ -759,12 +759,14 @@ __device__ __forceinline__ void dbcdef_tile(const DbCdefArgs& a, int tile_x, int
     }
 }
 
-// NT threads per tile, MIN_CTAS CTAs per SM.  The per-frame path runs 256
-// threads at 4 CTAs per SM (64 registers a thread), measured at least as fast
-// as 3 (80 registers) on 1080p and on 2560-, 2880- and 3840-wide frames
-// (1.5-2 % faster on the last two); 128 threads at 5 CTAs
-// per SM is the smaller-CTA shape (shorter barriers, about the same warps per
-// SM).
+// NT threads per tile, MIN_CTAS CTAs per SM.  The per-frame path runs 512
+// threads at 2 CTAs per SM for frames of up to two tiles per SM (see
+// launch_dbcdef_as()), else 256 threads at 4 CTAs per SM (64 registers a
+// thread), measured at least as fast as 3 (80 registers) on 1080p and on 2560-,
+// 2880- and 3840-wide frames (1.5-2 % faster on the last two); 128 threads at 5
+// CTAs per SM is the smaller-CTA shape (shorter barriers, about the same warps
+// per SM), which only the tuning selects: 13 % slower on the mix of frames
+// (3.37 against 2.97 ms for 64 frames), 15 % on a 4K frame (0.152, 0.132 ms).
 // DIRECT: a body that also writes the output of planes without restoration
 // (DirectPlane); the code for it measured 3 % slower on frames that have no
 // such plane, so it is a separate body.
